@@ -221,14 +221,15 @@ int clsph_gpu_set_launch_shape(clsph_gpu* h, int density_block, int forces_block
  * all modes give bit-identical results, they differ only in speed):
  *  WINDOW: one thread per particle walks its 2x2x2 window of cells and skips
  *    the particles in each neighbour cell's far half by their half-cell code;
- *  CELL_WARPS: one warp per occupied cell stages each neighbour cell's facing
- *    half in shared memory once for all of the cell's particles. The default;
+ *  CELL_WARPS: a team of warps per occupied cell stages the facing halves of
+ *    its neighbour cells in shared memory once for all of the cell's particles;
  *  PARTICLE_WARPS: one warp per particle tests 32 candidates at a time (for
  *    scenes too small to fill the GPU otherwise).
- * The density block size of clsph_gpu_set_launch_shape sets WINDOW's block
- * (64 or 128 threads; 256 runs as 128) and CELL_WARPS' staging tiles per
- * block (64 / 128 / 256 threads = 2 / 4 / 8 warps, each staging 32
- * candidates at a time); clsph_gpu_autotune tries every combination. */
+ * A new handle takes PARTICLE_WARPS for up to 14,000 particles and CELL_WARPS
+ * above. The density block size of clsph_gpu_set_launch_shape sets WINDOW's
+ * block (64 or 128 threads; 256 runs as 128) and the team of CELL_WARPS (64 /
+ * 128 / 256 threads = 2 / 4 / 8 warps); clsph_gpu_autotune tries every
+ * combination. */
 enum {
   CLSPH_SEARCH_WINDOW = 0,
   CLSPH_SEARCH_CELL_WARPS = 1,

@@ -81,6 +81,26 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
   return c;
 }
 
+// Density search of a new handle (clsph_gpu_set_neighbour_search,
+// clsph_gpu_set_launch_shape and clsph_gpu_autotune replace it). Measured
+// (density kernel, us; one warp per particle / teams of 4 / of 2 warps):
+//   water, spread on a floor: 4,096 particles 16 / 27 / 34; 10,000 23 / 29 / 38;
+//   20,000 37 / 34 / 42; 32,768 55 / 35 / 44; 65,536 102 / 53 / 52;
+//   131,072 196 / 77 / 75; 1,048,576 1549 / 395 / 309
+//   twice as many particles in a cell at rest: 10,000 29 / 39 / 58; 32,768
+//   69 / 49 / 68; 131,072 258 / 94 / 122; 1,048,576 - / 475 / 595
+// Few cells leave the chip idle unless a cell's work is spread wider; cells of
+// many particles keep four warps busy. Fluids whose 2h cell holds more than 50
+// particles at rest (38 at 20 particles within the radius, 76 at 40) also take
+// the larger lists: shared memory for 92 chunks lets 16 teams of two share an
+// SM, for 128 chunks 12 (1,048,576 particles of water: 0.309 against 0.346 ms).
+void choose_search(clsph_gpu* h) {
+  for (const Consts& c : h->consts_host)
+    if (!(8.f * c.h * c.h * c.h * c.rho0 <= 50.f * c.mass)) h->packed_cells = true;
+  h->search = h->n <= 14000u ? CLSPH_SEARCH_PARTICLE_WARPS : CLSPH_SEARCH_CELL_WARPS;
+  h->density_block = h->packed_cells || h->n <= 64000u ? 128 : 64;
+}
+
 }  // namespace
 
 int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
@@ -106,7 +126,7 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
   h->launch(K_GATHER, k_gather, dim3(blocks), dim3(kBlock), n, (const DevGrid*)h->grids,
             (const uint16_t*)h->scene_of, cctl, (const uint32_t*)h->keys,
             (const uint32_t*)h->vals, h->st[0], h->st[1], (const uint32_t*)h->ids[src_ids],
-            h->ids[dst_ids], h->ci, h->cell_list, h->step_counters + kCntCells);
+            h->ids[dst_ids], h->ci, h->cell_list, h->step_counters + kCntCells, h->planes);
   h->ids_sel = dst_ids;
   if (until <= CLSPH_STAGE_SORT) return 0;
   {
@@ -119,20 +139,27 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
                 (const float4*)h->st[1].pos, h->ci, (const Consts*)h->consts, h->aux, h->nlist,
                 h->ncount, h->nlist_cap, (const float4*)h->st[1].vel, h->frec, h->nb_start);
     };
-    // cell-warp mode: the block size sets the warps (cell staging tiles) per
-    // block, 2, 4 or 8, each with its own 32-candidate tile and buffers
-    auto cells = [&](auto kernel, int warps) {
-      h->launch(K_DENSITY, kernel, dim3(h->sm_count * (64 / warps)), dim3(warps * 32),
+    // cell mode: the block size sets the warps of the team that works on a cell, 2, 4 or 8
+    auto cells = [&](auto kernel, int k, int warps) {
+      uint32_t& resident = h->density_resident[k];
+      if (!resident) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, 0) != cudaSuccess || per_sm < 1)
+          per_sm = 1;
+        resident = (uint32_t)per_sm * h->sm_count;
+      }
+      h->launch(K_DENSITY, kernel, dim3(std::min(resident, n)), dim3(warps * 32),
                 n, (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, cctl,
-                (const uint32_t*)h->keys, (const float4*)h->st[1].pos, h->ci,
+                (const uint32_t*)h->keys, (const float4*)h->st[1].pos, (const uint32_t*)h->planes, h->ci,
                 (const Consts*)h->consts, h->aux, h->nlist, h->ncount, h->nlist_cap,
-                (const float4*)h->st[1].vel, h->frec, (const uint32_t*)h->cell_list,
+                (const float4*)h->st[1].vel, h->frec, (const uint2*)h->cell_list,
                 h->step_counters, h->nb_start);
     };
     if (h->search == CLSPH_SEARCH_CELL_WARPS) {
-      if (h->density_block == 64) cells(k_density_cells<2>, 2);
-      else if (h->density_block == 256) cells(k_density_cells<8>, 8);
-      else cells(k_density_cells<kCellWarps>, kCellWarps);
+      if (h->density_block == 256) cells(k_density_cells<CellTeamSmem<8, 128, 14>, 3>, 3, 8);
+      else if (h->density_block == 128) cells(k_density_cells<CellTeamSmem<4, 128, 14>, 7>, 2, 4);
+      else if (h->packed_cells) cells(k_density_cells<CellTeamSmem<2, 128, 14>, 12>, 1, 2);
+      else cells(k_density_cells<CellTeamSmem<2, 92, 11>, 16>, 0, 2);
     } else if (h->search == CLSPH_SEARCH_PARTICLE_WARPS) {
       h->launch(K_DENSITY, k_density_pwarp, dim3((n + kParticleWarps - 1) / kParticleWarps),
                 dim3(kParticleWarps * 32), n, (const DevGrid*)h->grids, (const uint16_t*)h->scene_of,
@@ -170,7 +197,11 @@ int clsph_host::launch_persistent(clsph_gpu* h, uint32_t substeps) {
     int per_sm = 0, coop = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
     if (!coop) return fail(CLSPH_ERR_CUDA, "persistent substeps: the device has no cooperative launch");
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_substeps_persistent, kPersistThreads, 0));
+    // (the attribute belongs to the current device)
+    CUDA_TRY(cudaFuncSetAttribute(k_substeps_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(PersistSmem)));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_substeps_persistent, kPersistThreads,
+                                                           sizeof(PersistSmem)));
     if (per_sm < 1) return fail(CLSPH_ERR_CUDA, "persistent substeps: no resident block fits an SM");
     h->persist_blocks = (uint32_t)per_sm * h->sm_count;
   }
@@ -198,6 +229,7 @@ int clsph_host::launch_persistent(clsph_gpu* h, uint32_t substeps) {
   a.ids[1] = h->ids[1];
   a.ci = h->ci;
   a.cell_list = h->cell_list;
+  a.planes = h->planes;
   a.consts = h->consts;
   a.aux = h->aux;
   a.nlist = h->nlist;
@@ -217,7 +249,7 @@ int clsph_host::launch_persistent(clsph_gpu* h, uint32_t substeps) {
     uint32_t sel = (uint32_t)h->ids_sel;
     void* args[] = {&a, &count, &sel};
     CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_substeps_persistent, dim3(h->persist_blocks),
-                                         dim3(kPersistThreads), args, 0, h->stream));
+                                         dim3(kPersistThreads), args, sizeof(PersistSmem), h->stream));
     ++h->launches;
     h->ids_sel ^= (int)(count & 1u);
     done += count;
@@ -448,6 +480,7 @@ int clsph_gpu_create_batched(const clsph_parameters* params, const clsph_kernel_
       return bail(rc);
   }
   h->ntiles = (n + kRadixTile - 1) / kRadixTile;
+  choose_search(h);
   uint32_t slots = 1024;
   while (slots < 2u * n) slots <<= 1;
   h->slots = slots;
@@ -456,7 +489,8 @@ int clsph_gpu_create_batched(const clsph_parameters* params, const clsph_kernel_
   if ((rc = dev_alloc(&h->aux, n)) || (rc = dev_alloc(&h->acc, n)) || (rc = dev_alloc(&h->frec, 2 * (size_t)n)) ||
       (rc = dev_alloc(&h->nlist, (size_t)h->nlist_cap * n)) || (rc = dev_alloc(&h->ncount, n)) ||
       (rc = dev_alloc(&h->nb_start, 27 * (size_t)n + 32)) ||  // + 32: any 5-bit cell index stays inside
-      (rc = dev_alloc(&h->cell_list, n)) || (rc = dev_alloc(&h->step_counters, kStepCounters)) ||
+      (rc = dev_alloc(&h->cell_list, n)) ||
+      (rc = dev_alloc(&h->planes, kHalfPlanes * (((size_t)n + 31) / 32))) || (rc = dev_alloc(&h->step_counters, kStepCounters)) ||
       (rc = dev_alloc(&h->keys, 2 * (size_t)n)) || (rc = dev_alloc(&h->vals, 2 * (size_t)n)) ||
       (rc = dev_alloc(&h->lookback, 4 * 256 * (size_t)h->ntiles)) ||
       (rc = dev_alloc(&h->digit_total, 4 * 256)) || (rc = dev_alloc(&h->ci.keys, slots)) ||
@@ -525,7 +559,7 @@ int clsph_gpu_destroy(clsph_gpu* h) {
     cudaFree(h->ids[s]);
   }
   void* bufs[] = {h->aux,      h->acc,      h->frec,      h->nlist,     h->ncount,      h->cell_list,
-                  h->nb_start,
+                  h->nb_start, h->planes,
                   h->step_counters, h->keys, h->vals,     h->lookback,    h->digit_total,
                   h->ci.keys,  h->ci.start, h->ci.end,    h->scene_of,    h->grids,
                   h->consts,   h->scene_h,  h->meshes,    h->bbox,        h->ctl,

@@ -131,7 +131,8 @@ struct clsph_gpu {
   uint32_t* nb_start = nullptr;   // [n][27] rows of the cells' neighbour starts (by first slot)
   uint32_t* ncount = nullptr;
   uint32_t nlist_cap = 64;
-  uint32_t* cell_list = nullptr;      // first sorted slot of every occupied cell
+  uint2* cell_list = nullptr;         // first sorted slot and sort key of every occupied cell
+  uint32_t* planes = nullptr;         // half codes of the sorted slots as bit planes (kHalfPlanes per 32)
   uint32_t* step_counters = nullptr;  // kStepCounters, zeroed every substep
   uint32_t* keys = nullptr;           // [2n]
   uint32_t* vals = nullptr;           // [2n]
@@ -144,9 +145,11 @@ struct clsph_gpu {
   unsigned long long* capped = nullptr;
   float4* aos_stage = nullptr;
 
-  // launch shapes chosen by clsph_gpu_autotune
+  // launch shapes (density: by the handle's size until clsph_gpu_autotune or a setter replaces them)
   int density_block = 128;
   int search = CLSPH_SEARCH_CELL_WARPS;  // neighbour search of the density kernel
+  bool packed_cells = false;  // some scene's fluid at rest has more than 50 particles in a 2h cell
+  uint32_t density_resident[4] = {};  // resident blocks of each form of the cell search (0: not yet asked)
   int forces_block = 128;
   uint32_t advect_blocks_per_sm = 8;
 

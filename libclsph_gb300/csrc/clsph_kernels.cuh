@@ -21,6 +21,8 @@
 // trip between kernels.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "clsph_common.cuh"
 
 namespace clsph {
@@ -657,6 +659,11 @@ static __global__ void __launch_bounds__(kRadixThreads)
                    spin_limit, withheld_tile, sm);
 }
 
+// Half codes as bit planes: word [g * kHalfPlanes + b] holds bit b of the half
+// codes of the 32 sorted slots of group g (written by k_gather, read by the
+// cell search).
+constexpr uint32_t kHalfPlanes = 6;
+
 // Gathers the state into sorted order (the stable scatter of sort.cl:41-59)
 // and records every cell's [start, end) in the cell index (the dense cell
 // table of sph_simulation.cpp:162-170 in compact form).
@@ -673,8 +680,9 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
                                              const uint32_t* __restrict__ keys_base,
                                              const uint32_t* __restrict__ vals_base, State src, State dst,
                                              const uint32_t* __restrict__ ids_src, uint32_t* __restrict__ ids_dst,
-                                             CellIndex ci, uint32_t* __restrict__ cell_list,
-                                             uint32_t* __restrict__ cell_count, GatherSmem& sm) {
+                                             CellIndex ci, uint2* __restrict__ cell_list,
+                                             uint32_t* __restrict__ cell_count, uint32_t* __restrict__ planes,
+                                             GatherSmem& sm) {
   auto& warp_base = sm.warp_base;
   uint32_t& block_base = sm.block_base;
   const uint32_t s = vb * blockDim.x + threadIdx.x;
@@ -684,11 +692,13 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
   const uint32_t* keys = keys_base + (size_t)sel * n;
   const uint32_t* perm = vals_base + (size_t)sel * n;
   bool first = false;
+  uint32_t key = 0u, code = 0u;
   if (s < n) {
     const uint32_t from = min(perm[s], n - 1u);  // in range even after a flagged sort stall
-    const uint32_t key = keys[s];
+    key = keys[s];
     float4 p = src.pos[from];
-    p.w = __uint_as_float(half_code(p, split.morton(key), grids[scene_of[s]]));
+    code = half_code(p, split.morton(key), grids[scene_of[s]]);
+    p.w = __uint_as_float(code);
     dst.pos[s] = p;
     dst.vel[s] = src.vel[from];
     dst.ivel[s] = src.ivel[from];
@@ -703,6 +713,13 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
       if (slot != 0xFFFFFFFFu) ci.end[slot] = s + 1;
     }
   }
+  uint32_t plane = 0u;  // the half codes of the warp's 32 slots as bit planes, for the cell search
+#pragma unroll
+  for (uint32_t b = 0; b < kHalfPlanes; ++b) {
+    const uint32_t v = __ballot_sync(0xFFFFFFFFu, (code >> b) & 1u);
+    if (lane == b) plane = v;
+  }
+  if (lane < kHalfPlanes && (s & ~31u) < n) planes[(size_t)(s >> 5) * kHalfPlanes + lane] = plane;
   const uint32_t bal = __ballot_sync(0xFFFFFFFFu, first);
   if (lane == 0) warp_base[warp] = __popc(bal);
   __syncthreads();
@@ -716,7 +733,7 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
     block_base = run ? atomicAdd(cell_count, run) : 0u;
   }
   __syncthreads();
-  if (first) cell_list[block_base + warp_base[warp] + __popc(bal & ((1u << lane) - 1u))] = s;
+  if (first) cell_list[block_base + warp_base[warp] + __popc(bal & ((1u << lane) - 1u))] = make_uint2(s, key);
   __syncthreads();  // the shared counts are read before the block's next use
 }
 
@@ -726,11 +743,11 @@ static __global__ void __launch_bounds__(kBlock)
              const uint32_t* __restrict__ keys_base,
              const uint32_t* __restrict__ vals_base, State src, State dst,
              const uint32_t* __restrict__ ids_src, uint32_t* __restrict__ ids_dst,
-             CellIndex ci, uint32_t* __restrict__ cell_list,
-             uint32_t* __restrict__ cell_count) {
+             CellIndex ci, uint2* __restrict__ cell_list,
+             uint32_t* __restrict__ cell_count, uint32_t* __restrict__ planes) {
   __shared__ GatherSmem sm;
   gather_block(blockIdx.x, n, grids, scene_of, ctl, keys_base, vals_base, src, dst, ids_src, ids_dst, ci,
-               cell_list, cell_count, sm);
+               cell_list, cell_count, planes, sm);
 }
 
 // ------------------------------------------------- density and forces
@@ -993,313 +1010,29 @@ __global__ void __launch_bounds__(BLOCK)
                   untagged ? max(kept, nlist_cap + 1u) : kept);
 }
 
-// ------------------------------------------------- density, one warp per cell
-// The warp takes one occupied cell at a time (dynamic work counter), looks up
-// the 27 cells around it once (lane k < 27: offset k in the reference's z, y,
-// x loop order; also stored as the cell's nb_start row) and holds the cell's
-// particles, two per lane. For each neighbour cell, in that order, that lies
-// in at least one particle's window (the union of the windows as a 27-bit
-// mask), it walks the cell's slots 32 at a time and stages the candidates
-// that face the own cell (the far half is skipped by half code), compacted by
-// ballot, which keeps their sorted order, into a tile in shared memory, with
-// coordinates relative to the own cell's centre and their negated squared
-// norm. A tile holds up to 32 candidates, of one cell or of consecutive
-// cells: it is tested before a block would overflow it and at the end of the
-// pass. A lane tests both its particles against every staged candidate with
-// three FMAs, 2 p'.q' - |q'|^2 >= |p'|^2 - R^2 (the squared distance with the
-// particle's part precomputed), sets the candidate's bit in the tile's hit
-// mask, and after the tile appends the hits' tags to the particle's buffer in
-// bit order, so each buffer holds the reference's visiting order. A particle
-// also tests candidates of cells outside its own window (those of the other
-// particles' windows); the exact test rejects them, as the reference's walk
-// over all 27 cells does. The survivors are then evaluated exactly per
-// particle, as in k_density.
-// (Packing the candidates into tiles, instead of testing each 32-slot block
-// on its own, cut the kernel's instructions by 8.5 % and its time by 6-8 %
-// on the 1M dam break; letting tiles span cells, without skipping a half of
-// the lanes whose particles' windows miss the tile's cell, cut another 5 %
-// of the instructions and 4-7 % of the time.)
-//
-// Rounding of the cull: cell-relative coordinates are within 3h of the
-// centre, so every intermediate of the test is below 50 h^2 and the four
-// roundings of each side stay below 3e-5 h^2, a fifth of the cull's margin
-// (R^2 = 1.0005 h^2); the test is conservative, and the exact evaluation
-// decides.
-// A buffer entry is a neighbour tag; cells of 2048 or more particles and full
-// buffers send the particle to the in-order rescan.
-constexpr int kCellWarps = 4;
-constexpr uint32_t kCellOffBits = kTagOffBits;
-
-// Per neighbour offset k (z, y, x order): the half-code bits a candidate of
-// that cell needs to face the own cell, facing_mask(o).
-struct OffsetMasks {
-  uint8_t m[27];
-};
-constexpr OffsetMasks make_offset_masks() {
-  OffsetMasks t{};
-  for (int k = 0; k < 27; ++k) {
-    const int o[3] = {k % 3 - 1, (k / 3) % 3 - 1, k / 9 - 1};
-    uint32_t cand = 0;
-    for (int a = 0; a < 3; ++a) {
-      if (o[a] < 0) cand |= 2u << (2 * a);
-      if (o[a] > 0) cand |= 1u << (2 * a);
-    }
-    t.m[k] = (uint8_t)cand;
-  }
-  return t;
-}
-__constant__ OffsetMasks kOffsetMasks = make_offset_masks();
-
+// ------------------------------------------------- density, one particle by a warp
+// The warp walks the particle's window cells in the reference's order, 32
+// candidates at a time (far halves skipped by half code, FMA cull), every
+// lane evaluates its candidate exactly, and the contributing terms are added
+// to the density one after another in lane order (ballot + shuffle), which is
+// the reference's visiting order; survivors append to the neighbour list in
+// the same order.
 __device__ __forceinline__ bool near_cull(const float4& p, const float4& q, float r2) {
   const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
   return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= r2;
 }
 
-// The cells of a particle's window as bits k < 27 (z, y, x order): on every
-// axis offset 0, and -1 / +1 where its half code has the lower / upper bit.
-// Bit k is set exactly when (code & facing_mask(-o)) == facing_mask(-o) for
-// the cell's offset o.
-__device__ __forceinline__ uint32_t window_cells(uint32_t code) {
-  const uint32_t ax = 2u | (code & 1u) | ((code << 1) & 4u);
-  const uint32_t ay = 2u | ((code >> 2) & 1u) | ((code >> 1) & 4u);
-  const uint32_t az = 2u | ((code >> 4) & 1u) | ((code >> 3) & 4u);
-  const uint32_t yx = ((ay & 1u) ? ax : 0u) | (ax << 3) | ((ay & 4u) ? ax << 6 : 0u);
-  return ((az & 1u) ? yx : 0u) | (yx << 9) | ((az & 4u) ? yx << 18 : 0u);
-}
-
-// survivor buffer per particle: 48 tags (40 with 8 warps, which keeps the
-// block within 48 KB of shared memory); fuller ones rescan
-template <int WARPS>
-struct DensitySmem {
-  static constexpr uint32_t kCap = WARPS >= 8 ? 40u : (uint32_t)kScanCap;
-  float4 stage[WARPS][32];
-  uint32_t stag[WARPS][32];
-  uint32_t starts[WARPS][32];
-  uint16_t cand[WARPS][kCap][64];
-};
-
-template <int WARPS>
-__device__ __forceinline__ void density_cells_warps(
-    uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
-    const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ keys_base, const float4* __restrict__ pos,
-    CellIndex ci, const Consts* __restrict__ consts, float4* __restrict__ aux_out, uint16_t* __restrict__ nlist,
-    uint32_t* __restrict__ ncount, uint32_t nlist_cap, const float4* __restrict__ vel,
-    float4* __restrict__ frec, const uint32_t* __restrict__ cell_list, uint32_t* __restrict__ counters,
-    uint32_t* __restrict__ nb_start, DensitySmem<WARPS>& sm) {
-  constexpr uint32_t kCap = DensitySmem<WARPS>::kCap;
-  auto& stage = sm.stage;
-  auto& stag = sm.stag;
-  auto& starts = sm.starts;
-  auto& cand = sm.cand;
-  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t ncells = counters[kCntCells];
-  const KeySplit split{ctl[kCtlShift]};
-  const uint32_t* keys = keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n;
-  for (;;) {
-    uint32_t cell = 0;
-    if (lane == 0) cell = atomicAdd(&counters[kCntWorkDensity], 1u);
-    cell = __shfl_sync(0xFFFFFFFFu, cell, 0);
-    if (cell >= ncells) break;
-    const uint32_t s0 = cell_list[cell];
-    const uint32_t key = split.morton(keys[s0]);
-    const uint32_t sc = scene_of[s0];
-    const uint32_t sbits = split.scene_bits(sc);
-    const uint32_t cx = compact_bits3(key), cy = compact_bits3(key >> 1), cz = compact_bits3(key >> 2);
-    const float cull_r2 = consts[sc].cull_r2;
-    const DevGrid& gr = grids[sc];
-    // the own cell's centre: the origin of the cull's coordinates
-    const float ox = gr.lo[0] + ((float)cx + 0.5f) * gr.cell, oy = gr.lo[1] + ((float)cy + 0.5f) * gr.cell,
-                oz = gr.lo[2] + ((float)cz + 0.5f) * gr.cell;
-    uint32_t nb_s = 0, nb_e = 0;
-    if (lane < 27u) {
-      const uint32_t x = cx + lane % 3u - 1u, y = cy + (lane / 3u) % 3u - 1u, z = cz + lane / 9u - 1u;
-      const uint2 r = cell_lookup(ci, morton3(x, y, z) | sbits);
-      nb_s = r.x;
-      nb_e = r.y;
-      nb_start[(size_t)s0 * 27u + lane] = nb_s;
-    }
-    starts[wid][lane] = nb_s;
-    __syncwarp();
-    const uint32_t own_e = __shfl_sync(0xFFFFFFFFu, nb_e, 13);
-    const bool wide = __any_sync(0xFFFFFFFFu, nb_e - nb_s >= (1u << kCellOffBits));
-    for (uint32_t base = s0; base < own_e; base += 64u) {
-      const uint32_t ia = base + lane, ib = base + 32u + lane;
-      const bool va = ia < own_e, vb = ib < own_e;
-      const float4 pa = va ? pos[ia] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 pb = vb ? pos[ib] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const uint32_t code_a = __float_as_uint(pa.w), code_b = __float_as_uint(pb.w);
-      // 2 p' and |p'|^2 - R^2 of both particles
-      const float ax = pa.x - ox, ay = pa.y - oy, az = pa.z - oz;
-      const float bx = pb.x - ox, by = pb.y - oy, bz = pb.z - oz;
-      const float a2x = 2.f * ax, a2y = 2.f * ay, a2z = 2.f * az;
-      const float b2x = 2.f * bx, b2y = 2.f * by, b2z = 2.f * bz;
-      const float ta = fmaf(ax, ax, fmaf(ay, ay, az * az)) - cull_r2;
-      const float tb = fmaf(bx, bx, fmaf(by, by, bz * bz)) - cull_r2;
-      uint32_t fa = wide ? kCap + 1u : 0u, fb = fa;
-      // the cells of the pass's windows (the union over its particles) in z,
-      // y, x order, each walked in 32-slot blocks; their facing candidates are
-      // packed into tiles of up to 32 (a tile is tested before a block would
-      // overflow it and at the end of the pass)
-      uint32_t rem = 0;
-      if (!wide)
-        rem = __reduce_or_sync(0xFFFFFFFFu, (va ? window_cells(code_a) : 0u) | (vb ? window_cells(code_b) : 0u));
-      uint32_t nt = 0;  // candidates in the tile
-      auto test_tile = [&]() {
-        const uint32_t m = nt;
-        // slots [m, 8 * ceil(m / 8)) hold a candidate no test accepts
-        if (m + lane < ((m + 7u) & ~7u)) stage[wid][m + lane] = make_float4(0.f, 0.f, 0.f, -INFINITY);
-        __syncwarp();
-        const float tak = va ? ta : INFINITY, tbk = vb ? tb : INFINITY;
-        // the a or b half of the lanes skips the tile when it holds no particle
-        const bool one = __any_sync(0xFFFFFFFFu, va), two = __any_sync(0xFFFFFFFFu, vb);
-        uint32_t ma = 0, mb = 0;
-        // eight candidates per step, each with its own constant bit
-        for (uint32_t t0 = 0; t0 < m; t0 += 8u) {
-          uint32_t ga = 0, gb = 0;
-#pragma unroll
-          for (uint32_t u = 0; u < 8u; ++u) {
-            const float4 r = stage[wid][t0 + u];
-            if (one && fmaf(a2x, r.x, fmaf(a2y, r.y, fmaf(a2z, r.z, r.w))) >= tak) ga |= 1u << u;
-            if (two && fmaf(b2x, r.x, fmaf(b2y, r.y, fmaf(b2z, r.z, r.w))) >= tbk) gb |= 1u << u;
-          }
-          ma |= ga << t0;
-          mb |= gb << t0;
-        }
-        // hits in candidate order
-        while (ma) {
-          const uint32_t t = __ffs(ma) - 1u;
-          ma &= ma - 1u;
-          if (fa < kCap) cand[wid][fa][lane] = (uint16_t)stag[wid][t];
-          ++fa;
-        }
-        while (mb) {
-          const uint32_t t = __ffs(mb) - 1u;
-          mb &= mb - 1u;
-          if (fb < kCap) cand[wid][fb][lane + 32u] = (uint16_t)stag[wid][t];
-          ++fb;
-        }
-        __syncwarp();
-        nt = 0;
-      };
-      while (rem) {
-        const uint32_t k = __ffs(rem) - 1u;
-        rem &= rem - 1u;
-        const uint32_t fm = kOffsetMasks.m[k];  // a candidate's half toward the own cell
-        const uint32_t s = __shfl_sync(0xFFFFFFFFu, nb_s, k), e = __shfl_sync(0xFFFFFFFFu, nb_e, k);
-        for (uint32_t cb = s; cb < e; cb += 32u) {
-          const uint32_t j = cb + lane;
-          float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-          bool f = false;
-          if (j < e) {
-            q = __ldg(&pos[j]);
-            f = (__float_as_uint(q.w) & fm) == fm;
-          }
-          const uint32_t bal = __ballot_sync(0xFFFFFFFFu, f);
-          const uint32_t cnt = __popc(bal);
-          if (nt + cnt > 32u) test_tile();  // the block would overflow the tile
-          if (f) {
-            const uint32_t at = nt + __popc(bal & lt);
-            const float qx = q.x - ox, qy = q.y - oy, qz = q.z - oz;
-            stage[wid][at] = make_float4(qx, qy, qz, -fmaf(qx, qx, fmaf(qy, qy, qz * qz)));
-            stag[wid][at] = (k << kCellOffBits) | (j - s);
-          }
-          nt += cnt;
-          if (nt == 32u) test_tile();
-        }
-      }
-      if (nt) test_tile();  // the end of the pass
-      auto finish = [&](uint32_t i, const float4& pi, uint32_t found, uint32_t col) {
-        const Consts& c = consts[sc];
-        const float hh = XMUL(c.h, c.h);
-        float rho = 0.f;
-        uint32_t kept = 0;
-        bool untagged = false;
-        auto visit = [&](uint32_t j, float4 pj, uint32_t tag) {
-          const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
-          const float rr = xnorm(d);
-          if (rr < c.h) {
-            rho = XADD(rho, poly6_term(rr, hh, c));
-            if (tag == kNoTag) untagged = true;
-            else if (kept < nlist_cap) __stcs(&nlist[(size_t)kept * n + i], (uint16_t)tag);
-            ++kept;
-          }
-        };
-        if (found <= kCap) {
-          // each survivor's position is loaded one survivor ahead
-          auto slot_at = [&](uint32_t k) {
-            const uint32_t tag = cand[wid][k][col];
-            return starts[wid][tag >> kCellOffBits] + (tag & ((1u << kCellOffBits) - 1u));
-          };
-          uint32_t tag = found ? (uint32_t)cand[wid][0][col] : 0u;
-          float4 pj = found ? __ldg(&pos[slot_at(0)]) : make_float4(0.f, 0.f, 0.f, 0.f);
-          for (uint32_t k = 0; k < found; ++k) {
-            const uint32_t kn = k + 1 < found ? k + 1 : k;
-            const uint32_t tagn = cand[wid][kn][col];
-            const float4 pn = __ldg(&pos[slot_at(kn)]);
-            visit(0u, pj, tag);
-            tag = tagn;
-            pj = pn;
-          }
-        } else {
-          const Window w = neighbour_window(pi, key, grids[sc]);
-          for_each_facing_candidate(w, key, sbits, ci, pos, [&](uint32_t j, float4 pj, uint32_t tag) {
-            if (near_cull(pi, pj, c.cull_r2)) visit(j, pj, tag);
-          });
-        }
-        density_outputs(i, n, rho, c, s0, pi, vel, aux_out, frec, ncount,
-                        untagged ? max(kept, nlist_cap + 1u) : kept);
-      };
-      if (va) finish(ia, pa, fa, lane);
-      if (vb) finish(ib, pb, fb, lane + 32u);
-      __syncwarp();
-    }
-    __syncwarp();
-  }
-}
-
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
-    k_density_cells(uint32_t n, const DevGrid* __restrict__ grids,
-                    const uint16_t* __restrict__ scene_of, const uint32_t* __restrict__ ctl,
-                    const uint32_t* __restrict__ keys_base, const float4* __restrict__ pos,
-                    CellIndex ci, const Consts* __restrict__ consts, float4* __restrict__ aux_out,
-                    uint16_t* __restrict__ nlist, uint32_t* __restrict__ ncount,
-                    uint32_t nlist_cap, const float4* __restrict__ vel,
-                    float4* __restrict__ frec, const uint32_t* __restrict__ cell_list,
-                    uint32_t* __restrict__ counters, uint32_t* __restrict__ nb_start) {
-  __shared__ DensitySmem<WARPS> sm;
-  density_cells_warps<WARPS>(n, grids, scene_of, ctl, keys_base, pos, ci, consts, aux_out, nlist, ncount,
-                             nlist_cap, vel, frec, cell_list, counters, nb_start, sm);
-}
-
-
-// Density + pressure + neighbour list with one warp per particle, for scenes
-// too small to fill the GPU with one thread per particle or one warp per
-// cell. The warp walks the particle's window cells in the reference's order,
-// 32 candidates at a time (far halves skipped by half code, FMA cull), every
-// lane evaluates its candidate exactly, and the contributing terms are added
-// to the density one after another in lane order (ballot + shuffle), which is
-// the reference's visiting order; survivors append to the neighbour list in
-// the same order.
-constexpr int kParticleWarps = 8;
-
-static __global__ void __launch_bounds__(kParticleWarps * 32)
-    k_density_pwarp(uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
-                    const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ keys_base,
-                    const float4* __restrict__ pos, CellIndex ci, const Consts* __restrict__ consts,
-                    float4* __restrict__ aux_out, uint16_t* __restrict__ nlist,
-                    uint32_t* __restrict__ ncount, uint32_t nlist_cap, const float4* __restrict__ vel,
-                    float4* __restrict__ frec, uint32_t* __restrict__ nb_start) {
+__device__ __forceinline__ void density_particle_warp(
+    uint32_t i, uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
+    const KeySplit& split, const uint32_t* __restrict__ keys, const float4* __restrict__ pos, const CellIndex& ci,
+    const Consts* __restrict__ consts, float4* __restrict__ aux_out, uint16_t* __restrict__ nlist,
+    uint32_t* __restrict__ ncount, uint32_t nlist_cap, const float4* __restrict__ vel, float4* __restrict__ frec,
+    uint32_t* __restrict__ nb_start) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= n) return;  // whole warps
-  const KeySplit split{ctl[kCtlShift]};
   const uint32_t sc = scene_of[i];
   const Consts& c = consts[sc];
   const uint32_t sbits = split.scene_bits(sc);
-  const uint32_t* keys = keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n;
   const uint32_t key = split.morton(keys[i]);
   const float4 pi = pos[i];
   const Window w = neighbour_window(pi, key, grids[sc]);
@@ -1361,6 +1094,431 @@ static __global__ void __launch_bounds__(kParticleWarps * 32)
   if (lane == 0)
     density_outputs(i, n, rho, c, own_start, pi, vel, aux_out, frec, ncount,
                     untagged ? max(kept, nlist_cap + 1u) : kept);
+}
+
+// Density + pressure + neighbour list with one warp per particle, for scenes
+// too small to fill the GPU with one thread per particle or one team per cell.
+constexpr int kParticleWarps = 8;
+
+static __global__ void __launch_bounds__(kParticleWarps * 32)
+    k_density_pwarp(uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
+                    const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ keys_base,
+                    const float4* __restrict__ pos, CellIndex ci, const Consts* __restrict__ consts,
+                    float4* __restrict__ aux_out, uint16_t* __restrict__ nlist,
+                    uint32_t* __restrict__ ncount, uint32_t nlist_cap, const float4* __restrict__ vel,
+                    float4* __restrict__ frec, uint32_t* __restrict__ nb_start) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;  // whole warps
+  const KeySplit split{ctl[kCtlShift]};
+  const uint32_t* keys = keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n;
+  density_particle_warp(i, n, grids, scene_of, split, keys, pos, ci, consts, aux_out, nlist, ncount, nlist_cap, vel,
+                        frec, nb_start);
+}
+
+// ------------------------------------------------- density, one team of warps per cell
+// A team of warps takes one occupied cell at a time (dynamic work counter):
+//  1. one warp looks up the 27 cells around it (lane k < 27: offset k in the
+//     reference's z, y, x loop order; also stored as the cell's nb_start row)
+//     and reads, from the half codes' bit planes, which of their particles
+//     face the own cell (the far half is skipped, as in k_density): the
+//     cell's candidates, whose tags it writes in visiting order;
+//  2. a particle in one octant of the cell needs 8 of the 27 lists (its 2 x 2
+//     x 2 window), 4 runs of consecutive candidates: the warp writes the
+//     numbers of each octant's chunks of eight candidates;
+//  3. all warps load the candidates' positions into the chunks: relative to
+//     the own cell's centre in units of h, in half precision, with the
+//     negated squared norm, candidate e beside candidate e + 4 so that one
+//     packed operation tests both;
+//  4. one lane per particle walks its octant's chunks: three packed FMAs and a
+//     packed compare test two candidates, 2 p'.q' - |q'|^2 >= |p'|^2 - R^2,
+//     and 32 candidates make one word of hit bits in shared memory, first
+//     candidate in the top bit;
+//  5. the lane walks its hit bits, which is the reference's visiting order,
+//     and evaluates each survivor exactly, as in k_density, with the next
+//     one's position in flight.
+// The first warp prepares the next cell (1, 2) before it waits for the
+// others. A chunk can hold candidates of a neighbouring list that the octant
+// doesn't need (they lie more than h away: the exact test drops them), and
+// one that two runs share is walked once. Particles that the lists don't
+// serve are done by a whole warp each (density_particle_warp): those on a
+// mid-plane of the cell, so in two octants; cells of up to kSparseCell
+// particles, for which the lists cost more than they save; lists longer than
+// the team's shared memory; and neighbours of a cell of 2048 or more
+// particles, which tags can't address.
+//
+// Bound: instruction issue, half of it the exact evaluation. 1,048,576
+// particles spread over a floor (29,552 cells, a quarter of them of one or
+// two particles): 212 M warp instructions, 60 % of the issue slots, 0.309 ms,
+// against 313 M and 0.454 ms for the form before, one warp per cell that
+// tested each of its 64 particles against all 512 candidates in FP32; the
+// same on the h/2 lattice: 0.235 ms against 0.359. Of the 212 M: the cell's
+// look-up and the outputs 38 M, candidates 24 M, culls 38 M (an octant's 216
+// candidates instead of 512, two per operation), exact evaluation 112 M.
+// Staging with FP32 positions streamed per neighbour list and compacted by
+// ballot took 104 M (each list's far half is read and dropped, and a list
+// rarely fills its warps); planes cost one bit per particle and axis half.
+//
+// Rounding of the cull, in units of h. Candidates that matter lie within 1 of
+// a particle inside the own cell: |p'| <= sqrt(3), |q'| < 2.74, |q'|^2 < 7.5.
+// Rounding p' and q' to 11 bits moves 2 p'.q' by at most 2 (2.74 * 4.3e-4 +
+// 1.74 * 8.5e-4) < 5.4e-3; storing |q'|^2 and the three packed FMAs round
+// values below 8, at most 2^-9 each: 7.9e-3 in all. |p'|^2 - R^2 is rounded
+// down. So every candidate within h passes with R^2 = 1.015 > 1 + 1.33e-2;
+// the exact evaluation decides.
+constexpr float kCellCullR2 = 1.015f;
+constexpr uint32_t kCellOffBits = kTagOffBits;
+
+// Per neighbour offset k (z, y, x order): the half-code bits a candidate of
+// that cell needs to face the own cell, facing_mask(o).
+struct OffsetMasks {
+  uint8_t m[27];
+};
+constexpr OffsetMasks make_offset_masks() {
+  OffsetMasks t{};
+  for (int k = 0; k < 27; ++k) {
+    const int o[3] = {k % 3 - 1, (k / 3) % 3 - 1, k / 9 - 1};
+    uint32_t cand = 0;
+    for (int a = 0; a < 3; ++a) {
+      if (o[a] < 0) cand |= 2u << (2 * a);
+      if (o[a] > 0) cand |= 1u << (2 * a);
+    }
+    t.m[k] = (uint8_t)cand;
+  }
+  return t;
+}
+__constant__ OffsetMasks kOffsetMasks = make_offset_masks();
+
+// The cells of a particle's window as bits k < 27 (z, y, x order): on every
+// axis offset 0, and -1 / +1 where its half code has the lower / upper bit.
+// Bit k is set exactly when (code & facing_mask(-o)) == facing_mask(-o) for
+// the cell's offset o.
+__device__ __forceinline__ uint32_t window_cells(uint32_t code) {
+  const uint32_t ax = 2u | (code & 1u) | ((code << 1) & 4u);
+  const uint32_t ay = 2u | ((code >> 2) & 1u) | ((code >> 1) & 4u);
+  const uint32_t az = 2u | ((code >> 4) & 1u) | ((code >> 3) & 4u);
+  const uint32_t yx = ((ay & 1u) ? ax : 0u) | (ax << 3) | ((ay & 4u) ? ax << 6 : 0u);
+  return ((az & 1u) ? yx : 0u) | (yx << 9) | ((az & 4u) ? yx << 18 : 0u);
+}
+
+// A cell of at most this many particles is done by a warp per particle.
+constexpr uint32_t kSparseCell = 4;
+
+// Shared memory of one team of WARPS warps: CHUNKS chunks for a cell's
+// candidates (512, 64 chunks, on the h/2 lattice), WORDS mask words for an
+// octant's (216, 7 words, and up to a chunk more per window row).
+template <int WARPS, int CHUNKS, int WORDS>
+struct CellTeamSmem {
+  static constexpr int kWarps = WARPS;
+  static constexpr uint32_t kChunks = CHUNKS, kWords = WORDS;
+  static_assert(CHUNKS <= 256, "chunk numbers are bytes");
+  uint4 chunk[CHUNKS][5];  // four pairs of four halves; eight 16-bit tags
+  uint4 no_chunk[4];       // a chunk that never hits
+  uint32_t mask[WARPS][WORDS][32];
+  uint16_t pend[8 * CHUNKS];  // the next cell's candidates: their tags in visiting order
+  // two sets of what is known of a cell: one is made while the other is read
+  struct Cell {
+    float4 origin;           // its centre and 1 / h
+    uint32_t slot_of[32];    // slot minus tag of neighbour k's particles
+    uint32_t seq[8][WORDS];  // an octant's chunk numbers, four to a word, first in the top byte
+    uint32_t chunks[8];      // and their count
+    uint32_t scene, first, count;  // its particles
+    uint32_t candidates;     // kNoLists: the lists don't serve it; kNoCell: no cell left
+  } cell[2];
+};
+constexpr uint32_t kNoLists = 0xFFFFFFFEu, kNoCell = 0xFFFFFFFFu;
+
+// The slots of word `w` of the planes in [s, e) that have all of `need`.
+__device__ __forceinline__ uint32_t facing_slots(const uint32_t* __restrict__ planes, uint32_t w, uint32_t s,
+                                                 uint32_t e, uint32_t need) {
+  const uint32_t* p = planes + (size_t)w * kHalfPlanes;
+  uint32_t m = 0xFFFFFFFFu;
+#pragma unroll
+  for (uint32_t b = 0; b < kHalfPlanes; b += 2) {  // an axis needs at most one of its two bits
+    const uint32_t both = (need >> b) & 3u;
+    if (both) m &= __ldg(&p[b + (both >> 1)]);
+  }
+  const uint32_t w0 = 32u * w;
+  if (s > w0) m &= 0xFFFFFFFFu << (s - w0);
+  if (e < w0 + 32u) m &= (1u << (e - w0)) - 1u;
+  return m;
+}
+
+template <class Team>
+__device__ __forceinline__ void density_cells_team(
+    uint32_t n, const DevGrid* __restrict__ grids, const uint32_t* __restrict__ ctl,
+    const uint16_t* __restrict__ scene_of, const uint32_t* __restrict__ keys_base, const float4* __restrict__ pos,
+    const uint32_t* __restrict__ planes, const CellIndex& ci, const Consts* __restrict__ consts,
+    float4* __restrict__ aux_out, uint16_t* __restrict__ nlist, uint32_t* __restrict__ ncount, uint32_t nlist_cap,
+    const float4* __restrict__ vel, float4* __restrict__ frec, const uint2* __restrict__ cell_list,
+    uint32_t* __restrict__ counters, uint32_t* __restrict__ nb_start, Team& sm, uint32_t wid, uint32_t team,
+    uint32_t teams, uint32_t barrier_id) {
+  constexpr uint32_t kWarps = Team::kWarps, kWords = Team::kWords;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t lt = (1u << lane) - 1u;
+  auto team_sync = [&]() {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(barrier_id), "n"(kWarps * 32) : "memory");
+  };
+  constexpr uint32_t kNever = 0xFC00u;  // -infinity in half precision: a squared norm that no test accepts
+  if (wid == 0 && lane < 4u) sm.no_chunk[lane] = make_uint4(0u, 0u, 0u, kNever * 0x10001u);
+  const uint32_t ncells = counters[kCntCells];
+  const KeySplit split{ctl[kCtlShift]};
+  auto by_warp = [&](uint32_t i) {
+    density_particle_warp(i, n, grids, scene_of, split, keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n, pos, ci,
+                          consts, aux_out, nlist, ncount, nlist_cap, vel, frec, nb_start);
+  };
+  // the last warp, which has the fewest particles, looks the next cell up; the first two cells have fixed
+  // numbers, the others come from the work counter, and both are loaded a cell ahead
+  const bool fetcher = wid == kWarps - 1u;
+  uint32_t ticket = team;
+  uint2 entry = make_uint2(0u, 0u);
+  bool have = false;
+  auto load_entry = [&]() {
+    have = ticket < ncells;
+    if (have) entry = __ldg(&cell_list[ticket]);
+  };
+  if (fetcher) {
+    load_entry();
+    ticket += teams;
+  }
+  for (uint32_t par = 0;; par ^= 1u) {
+    typename Team::Cell& cell = sm.cell[par];
+    if (fetcher && !have) {
+      if (lane == 0) cell.candidates = kNoCell;
+    } else if (fetcher) {
+      const uint2 own = entry;
+      const uint32_t key = split.morton(own.y);
+      uint32_t s = 0, e = 0;
+      if (lane < 27u) {
+        const uint32_t x = compact_bits3(key) + lane % 3u - 1u, y = compact_bits3(key >> 1) + (lane / 3u) % 3u - 1u,
+                       z = compact_bits3(key >> 2) + lane / 9u - 1u;
+        const uint2 r = cell_lookup(ci, morton3(x, y, z) | (own.y ^ key));
+        s = lane == 13u ? own.x : r.x;  // (a flagged sort stall can leave the index with another start)
+        e = r.y;
+        nb_start[(size_t)own.x * 27u + lane] = s;
+      }
+      load_entry();
+      uint32_t next = 0;
+      if (lane == 0) next = atomicAdd(&counters[kCntWorkDensity], 1u);
+      ticket = __shfl_sync(0xFFFFFFFFu, next, 0) + 2u * teams;
+      const uint32_t own_e = __shfl_sync(0xFFFFFFFFu, e, 13);
+      const uint32_t count = own_e > own.x ? own_e - own.x : 0u;
+      uint32_t candidates = kNoLists;
+      if (!__any_sync(0xFFFFFFFFu, e - s >= (1u << kCellOffBits)) && count > kSparseCell) {
+        // the candidates of list k as bits, in up to three words of the planes (more are counted and read again)
+        const uint32_t need = kOffsetMasks.m[min(lane, 26u)];
+        const uint32_t w0 = s >> 5, words = e > s && lane != 13u ? ((e - 1u) >> 5) - w0 + 1u : 0u;
+        uint32_t m[3];
+#pragma unroll
+        for (uint32_t w = 0; w < 3u; ++w) m[w] = w < words ? facing_slots(planes, w0 + w, s, e, need) : 0u;
+        if (count <= 32u) {  // only the neighbour cells in its particles' windows
+          uint32_t any = 0;
+          if (lane < kHalfPlanes)
+            for (uint32_t w = own.x >> 5; w <= (own_e - 1u) >> 5; ++w) any |= facing_slots(planes, w, own.x, own_e, 1u << lane);
+          if (!((window_cells(__ballot_sync(0xFFFFFFFFu, any != 0u)) >> lane) & 1u)) m[0] = m[1] = m[2] = 0u;
+        }
+        uint32_t size = lane == 13u ? count : __popc(m[0]) + __popc(m[1]) + __popc(m[2]);
+        for (uint32_t w = 3; w < words; ++w) size += __popc(facing_slots(planes, w0 + w, s, e, need));
+        uint32_t end = size;
+#pragma unroll
+        for (uint32_t d = 1; d < 32u; d <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, end, d);
+          if (lane >= d) end += y;
+        }
+        const uint32_t begin = end - size;
+        const uint32_t all = __shfl_sync(0xFFFFFFFFu, end, 26);
+        if (all <= 8u * Team::kChunks) {
+          candidates = all;
+          const uint32_t own_at = __shfl_sync(0xFFFFFFFFu, begin, 13);
+          for (uint32_t j = lane; j < count; j += 32u) sm.pend[own_at + j] = (uint16_t)((13u << kCellOffBits) + j);
+          uint32_t tag = (lane << kCellOffBits) + 32u * w0 - s;  // of the first word's first slot
+          uint32_t at = begin;
+          for (uint32_t w = 2u; at < end && lane != 13u;) {
+            while (m[0] == 0u) {
+              m[0] = m[1];
+              m[1] = m[2];
+              ++w;
+              m[2] = w < words ? facing_slots(planes, w0 + w, s, e, need) : 0u;
+              tag += 32u;
+            }
+            sm.pend[at++] = (uint16_t)(tag + __ffs(m[0]) - 1u);
+            m[0] &= m[0] - 1u;
+          }
+          // octant o's chunks in visiting order: lane (o, r) appends those of window row r, two lists side by
+          // side, without a chunk that an earlier row shares
+          const uint32_t o = lane >> 2, r = lane & 3u;
+          const uint32_t k = (o & 1u) + 3u * (((o >> 1) & 1u) + (r & 1u)) + 9u * ((o >> 2) + (r >> 1));
+          const uint32_t a = __shfl_sync(0xFFFFFFFFu, begin, k), b = __shfl_sync(0xFFFFFFFFu, end, k + 1u);
+          uint32_t c0 = a >> 3;
+          const uint32_t c1 = b > a ? (b + 7u) >> 3 : 0u;  // chunks [c0, c1)
+          uint32_t seen = c1;
+#pragma unroll
+          for (uint32_t d = 1; d < 4u; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, seen, d, 4);
+            if (r >= d) seen = max(seen, y);
+          }
+          const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, seen, 1, 4);
+          if (r) c0 = max(c0, before);
+          const uint32_t cnt = c1 > c0 ? c1 - c0 : 0u;
+          uint32_t last = cnt;
+#pragma unroll
+          for (uint32_t d = 1; d < 4u; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, last, d, 4);
+            if (r >= d) last += y;
+          }
+          uint8_t* out = reinterpret_cast<uint8_t*>(cell.seq[o]);
+          uint32_t i = last - cnt;
+          for (uint32_t c = c0; c < c1 && i < 4u * kWords; ++c, ++i) out[i ^ 3u] = (uint8_t)c;
+          if (r == 3u) cell.chunks[o] = last;
+        }
+      }
+      cell.slot_of[lane] = s - (lane << kCellOffBits);
+      if (lane == 0) {
+        const uint32_t sc = split.shift >= 32u ? 0u : own.y >> split.shift;
+        const DevGrid& g = grids[sc];
+        cell.origin = make_float4(g.lo[0] + ((float)compact_bits3(key) + 0.5f) * g.cell,
+                                  g.lo[1] + ((float)compact_bits3(key >> 1) + 0.5f) * g.cell,
+                                  g.lo[2] + ((float)compact_bits3(key >> 2) + 0.5f) * g.cell, 1.f / consts[sc].h);
+        cell.scene = sc;
+        cell.first = own.x;
+        cell.count = count;
+        cell.candidates = candidates;
+      }
+    }
+    team_sync();
+    const uint32_t candidates = cell.candidates, first = cell.first, count = cell.count;
+    if (candidates == kNoCell) break;
+    if (candidates == kNoLists) {
+      for (uint32_t q = wid; q < count; q += kWarps) by_warp(first + q);
+      continue;
+    }
+    const float4 org = cell.origin;
+    constexpr uint32_t kAhead = 4;  // candidates in flight per thread
+    for (uint32_t e0 = 32u * wid + lane; e0 < candidates; e0 += 32u * kWarps * kAhead) {
+      uint32_t tag[kAhead];
+      float4 q[kAhead];
+#pragma unroll
+      for (uint32_t u = 0; u < kAhead; ++u) {
+        const uint32_t e = min(e0 + 32u * kWarps * u, candidates - 1u);
+        tag[u] = sm.pend[e];
+        q[u] = __ldg(&pos[cell.slot_of[tag[u] >> kCellOffBits] + tag[u]]);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kAhead; ++u) {
+        const uint32_t e = e0 + 32u * kWarps * u;
+        if (e >= candidates) break;
+        const float x = (q[u].x - org.x) * org.w, y = (q[u].y - org.y) * org.w, z = (q[u].z - org.z) * org.w;
+        uint4* c = sm.chunk[e >> 3];
+        __half* h = reinterpret_cast<__half*>(&c[e & 3u]) + ((e >> 2) & 1u);
+        h[0] = __float2half_rn(x);
+        h[2] = __float2half_rn(y);
+        h[4] = __float2half_rn(z);
+        h[6] = __float2half_rn(-fmaf(x, x, fmaf(y, y, z * z)));
+        reinterpret_cast<uint16_t*>(&c[4])[~e & 7u] = (uint16_t)tag[u];
+      }
+    }
+    if (wid == 0 && lane < (0u - candidates & 7u)) {  // the last chunk's free places
+      const uint32_t e = candidates + lane;
+      reinterpret_cast<uint16_t*>(&sm.chunk[e >> 3][e & 3u])[6u + ((e >> 2) & 1u)] = (uint16_t)kNever;
+    }
+    team_sync();
+    const Consts& c = consts[cell.scene];
+    for (uint32_t base = 32u * wid; base < count; base += 32u * kWarps) {
+      const bool valid = base + lane < count;
+      const uint32_t i = first + (valid ? base + lane : 0u);
+      const float4 pi = pos[i];
+      const uint32_t code = __float_as_uint(pi.w);
+      const float x = (pi.x - org.x) * org.w, y = (pi.y - org.y) * org.w, z = (pi.z - org.z) * org.w;
+      // the particle's octant, from its upper-half bits when each axis has exactly one
+      const uint32_t up = (code >> 1) & 0x15u;
+      const uint32_t o = (up & 1u) | ((up >> 1) & 2u) | ((up >> 2) & 4u);
+      uint32_t nc = cell.chunks[o];
+      const bool served = valid && ((code ^ up) & 0x15u) == 0x15u &&
+                          fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) < 1.25f && nc <= 4u * kWords;
+      if (!served) nc = 0u;
+      const uint32_t nw = (__reduce_max_sync(0xFFFFFFFFu, nc) + 3u) >> 2;
+      const __half2 px = __float2half2_rn(2.f * x), py = __float2half2_rn(2.f * y), pz = __float2half2_rn(2.f * z);
+      const __half2 pt = __half2half2(__float2half_rd(fmaf(x, x, fmaf(y, y, z * z)) - kCellCullR2));
+      const uint32_t* seq = cell.seq[o];
+      uint32_t* mask = &sm.mask[wid][0][lane];
+      uint32_t found = 0;
+      for (uint32_t w = 0; w < nw; ++w) {
+        const uint32_t ids = seq[w];
+        uint32_t acc = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+          const uint4* ch = 4u * w + q < nc ? sm.chunk[(ids >> (24u - 8u * q)) & 255u] : sm.no_chunk;
+#pragma unroll
+          for (uint32_t u = 0; u < 4u; ++u) {
+            const uint4 v = ch[u];
+            auto h2 = [](uint32_t b) { return *reinterpret_cast<const __half2*>(&b); };
+            const __half2 t = __hfma2(px, h2(v.x), __hfma2(py, h2(v.y), __hfma2(pz, h2(v.z), h2(v.w))));
+            acc |= __hge2_mask(t, pt) & (0x80008000u >> (4u * q + u));
+          }
+        }
+        // halves to candidate order: the upper half's nibble of each chunk after the lower half's
+        uint32_t m = __byte_perm(acc, 0u, 0x1302);
+        m ^= ((m ^ (m >> 4)) & 0x00F000F0u) * 17u;
+        mask[32u * w] = m;
+        found += __popc(m);
+      }
+      const float hh = XMUL(c.h, c.h);
+      float rho = 0.f;
+      uint32_t kept = 0;
+      uint16_t* list = nlist + i;
+      uint32_t m = 0, ids = 0, w = 0;
+      auto next = [&](uint32_t& tag) {  // the next survivor's tag and position
+        while (m == 0u) {
+          m = mask[32u * w];
+          ids = seq[w];
+          ++w;
+        }
+        const uint32_t b = 31u - __clz(m);
+        m ^= 1u << b;
+        tag = reinterpret_cast<const uint16_t*>(&sm.chunk[(ids >> (b & 24u)) & 255u][4])[b & 7u];
+        return __ldg(&pos[cell.slot_of[tag >> kCellOffBits] + tag]);
+      };
+      uint32_t tag = 0;
+      float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (found) pj = next(tag);
+      for (uint32_t k = 0; k < found;) {
+        uint32_t tagn = 0;
+        float4 pn = pj;
+        if (++k < found) pn = next(tagn);
+        const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
+        const float rr = xnorm(d);
+        if (rr < c.h) {
+          rho = XADD(rho, poly6_term(rr, hh, c));
+          if (kept < nlist_cap) __stcs(list, (uint16_t)tag);
+          list += n;
+          ++kept;
+        }
+        tag = tagn;
+        pj = pn;
+      }
+      if (served) density_outputs(i, n, rho, c, first, pi, vel, aux_out, frec, ncount, kept);
+      uint32_t rest = __ballot_sync(0xFFFFFFFFu, valid && !served);
+      while (rest) {
+        by_warp(first + base + __ffs(rest) - 1u);
+        rest &= rest - 1u;
+      }
+    }
+  }
+}
+
+template <class Team, int BLOCKS>
+__global__ void __launch_bounds__(Team::kWarps * 32, BLOCKS)
+    k_density_cells(uint32_t n, const DevGrid* __restrict__ grids,
+                    const uint16_t* __restrict__ scene_of, const uint32_t* __restrict__ ctl,
+                    const uint32_t* __restrict__ keys_base, const float4* __restrict__ pos,
+                    const uint32_t* __restrict__ planes, CellIndex ci, const Consts* __restrict__ consts,
+                    float4* __restrict__ aux_out, uint16_t* __restrict__ nlist, uint32_t* __restrict__ ncount,
+                    uint32_t nlist_cap, const float4* __restrict__ vel,
+                    float4* __restrict__ frec, const uint2* __restrict__ cell_list,
+                    uint32_t* __restrict__ counters, uint32_t* __restrict__ nb_start) {
+  __shared__ Team sm;
+  density_cells_team(n, grids, ctl, scene_of, keys_base, pos, planes, ci, consts, aux_out, nlist, ncount, nlist_cap, vel,
+                     frec, cell_list, counters, nb_start, sm, threadIdx.x >> 5, blockIdx.x, gridDim.x, 1u);
 }
 
 // Per-pair hook of k_forces (the learned stepper gathers its neighbour

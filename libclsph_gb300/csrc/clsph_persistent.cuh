@@ -6,7 +6,7 @@
 // turn, S substeps per launch, with a grid-wide barrier between phases:
 //   grid set-up (block 0) + cell-index clear | keys | digit counts |
 //   radix passes (tiles by ticket, decoupled look-back) | gather |
-//   density (one warp per occupied cell, 8 per block) | forces | advection
+//   density (two warps per occupied cell, 4 teams a block) | forces | advection
 // Each phase is the block-level body of the corresponding kernel of
 // clsph_kernels.cuh, so the results are those of the launched substeps bit
 // for bit. The barrier is a counter and a generation word in device memory;
@@ -40,7 +40,8 @@ struct PersistArgs {
   State st[2];
   uint32_t* ids[2];
   CellIndex ci;
-  uint32_t* cell_list;
+  uint2* cell_list;
+  uint32_t* planes;
   const Consts* consts;
   float4* aux;
   uint16_t* nlist;
@@ -55,15 +56,18 @@ struct PersistArgs {
   uint32_t barrier_limit, withheld_block;  // grid barrier bound and test hook
 };
 
+using PersistTeam = CellTeamSmem<2, 128, 14>;
+
 union PersistSmem {
   RadixSmem radix;
   uint32_t hist[4][256];
-  DensitySmem<8> dens;
+  PersistTeam dens[kPersistThreads / 64];  // one team of two warps for each 64 threads
   GatherSmem gather;
   BboxSmem bbox;
   uint32_t word;
 };
-static_assert(sizeof(PersistSmem) <= 48 * 1024, "static shared memory of the persistent kernel");
+// dynamic shared memory: three resident blocks of the SM's 227 KB
+static_assert(sizeof(PersistSmem) <= 74 * 1024, "shared memory of the persistent kernel");
 
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
@@ -109,7 +113,8 @@ __device__ __forceinline__ bool grid_barrier(const PersistArgs& a, uint32_t& ok_
 // three resident blocks per SM (24 warps): at most 85 registers per thread
 static __global__ void __launch_bounds__(kPersistThreads, 3)
     k_substeps_persistent(PersistArgs a, uint32_t substeps, uint32_t ids_sel0) {
-  __shared__ PersistSmem sm;
+  extern __shared__ __align__(16) unsigned char persist_smem[];
+  PersistSmem& sm = *reinterpret_cast<PersistSmem*>(persist_smem);
   __shared__ uint32_t ok_s;
   const uint32_t n = a.n;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,11 +144,13 @@ static __global__ void __launch_bounds__(kPersistThreads, 3)
     }
     for (uint32_t vb = blockIdx.x; vb < nblk; vb += gridDim.x)
       gather_block(vb, n, a.grids, a.scene_of, a.ctl, a.keys, a.vals, a.st[0], a.st[1], a.ids[src_ids],
-                   a.ids[src_ids ^ 1u], a.ci, a.cell_list, a.step_counters + kCntCells, sm.gather);
+                   a.ids[src_ids ^ 1u], a.ci, a.cell_list, a.step_counters + kCntCells, a.planes, sm.gather);
     if (!grid_barrier(a, ok_s)) return;
-    density_cells_warps<8>(n, a.grids, a.scene_of, a.ctl, a.keys, a.st[1].pos, a.ci, a.consts, a.aux, a.nlist,
-                           a.ncount, a.nlist_cap, a.st[1].vel, a.frec, a.cell_list, a.step_counters, a.nb_start,
-                           sm.dens);
+    density_cells_team(n, a.grids, a.ctl, a.scene_of, a.keys, a.st[1].pos, a.planes, a.ci, a.consts, a.aux, a.nlist,
+                       a.ncount, a.nlist_cap, a.st[1].vel, a.frec, a.cell_list, a.step_counters, a.nb_start,
+                       sm.dens[threadIdx.x >> 6], (threadIdx.x >> 5) & 1u,
+                       blockIdx.x * (kPersistThreads / 64u) + (threadIdx.x >> 6), gridDim.x * (kPersistThreads / 64u),
+                       1u + (threadIdx.x >> 6));
     if (!grid_barrier(a, ok_s)) return;
     for (uint32_t i = gtid; i < n; i += gstride)
       forces_particle(i, n, a.grids, a.scene_of, a.ctl, a.keys, a.st[1], a.aux, a.ci, a.consts, a.nlist, a.ncount,
