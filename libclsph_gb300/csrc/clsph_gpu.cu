@@ -78,6 +78,7 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
   // rounding of the cell-relative cull (k_density_cells) and far above that
   // of the direct differences; the exact test decides
   c.cull_r2 = p.h * p.h * 1.0005f;
+  c.plain_h = p.h >= 0x1p-20f && p.h <= 0x1p20f;
   return c;
 }
 
@@ -124,7 +125,7 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
               h->radix_withheld_tile);
   const int src_ids = h->ids_sel, dst_ids = h->ids_sel ^ 1;
   h->launch(K_GATHER, k_gather, dim3(blocks), dim3(kBlock), n, (const DevGrid*)h->grids,
-            (const uint16_t*)h->scene_of, cctl, (const uint32_t*)h->keys,
+            (const uint16_t*)h->scene_of, h->ctl, (const uint32_t*)h->keys,
             (const uint32_t*)h->vals, h->st[0], h->st[1], (const uint32_t*)h->ids[src_ids],
             h->ids[dst_ids], h->ci, h->cell_list, h->step_counters + kCntCells, h->planes);
   h->ids_sel = dst_ids;

@@ -130,7 +130,7 @@ struct clsph_gpu {
   uint16_t* nlist = nullptr;      // [nlist_cap][n] neighbour tags (visiting order)
   uint32_t* nb_start = nullptr;   // [n][27] rows of the cells' neighbour starts (by first slot)
   uint32_t* ncount = nullptr;
-  uint32_t nlist_cap = 64;
+  uint32_t nlist_cap = 96;
   uint2* cell_list = nullptr;         // first sorted slot and sort key of every occupied cell
   uint32_t* planes = nullptr;         // half codes of the sorted slots as bit planes (kHalfPlanes per 32)
   uint32_t* step_counters = nullptr;  // kStepCounters, zeroed every substep

@@ -23,6 +23,8 @@
 
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "clsph_common.cuh"
 
 namespace clsph {
@@ -72,8 +74,13 @@ __host__ __device__ __forceinline__ uint32_t sorted_sel(uint32_t maxkey) {
 }
 
 // Sort control block of a substep (device memory): [0] largest key,
-// [1] Morton bits (widest grid of all scenes), [2] scene bits.
-enum : int { kCtlMaxKey = 0, kCtlShift = 1, kCtlSceneBits = 2, kCtlWords = 8 };
+// [1] Morton bits (widest grid of all scenes), [2] scene bits, [3] nonzero when
+// some coordinate is nonzero but below kTinyCoordinate (k_gather).
+enum : int { kCtlMaxKey = 0, kCtlShift = 1, kCtlSceneBits = 2, kCtlTiny = 3, kCtlWords = 8 };
+
+// Differences of coordinates of at least this size are 0 or at least 2^-99,
+// as div_rn_normal needs.
+constexpr float kTinyCoordinate = 0x1p-76f;
 
 // Scene bits of a sort key and its Morton part.
 struct KeySplit {
@@ -94,6 +101,7 @@ struct Consts {
   float gx, gy, gz;
   float poly6, grad6, lap6, spiky, visc, spiky_zero;
   float cull_r2;  // conservative h^2 for the FMA cull test
+  uint32_t plain_h;  // h in [2^-20, 2^20]: near_norm and the short quotients are exact
 };
 
 struct State {
@@ -241,6 +249,7 @@ __device__ __forceinline__ void grid_setup_block(uint32_t* __restrict__ bbox_all
   __syncthreads();
   if (threadIdx.x == 0) {
     ctl[kCtlMaxKey] = 0u;
+    ctl[kCtlTiny] = 0u;
     ctl[kCtlShift] = shift_s;
     // scene bits above the Morton bits must fit in 32 (batched scenes)
     if (shift_s + ctl[kCtlSceneBits] > 32u) atomicOr(status, kFlagGridOverflow);
@@ -676,7 +685,7 @@ struct GatherSmem {
 
 __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevGrid* __restrict__ grids,
                                              const uint16_t* __restrict__ scene_of,
-                                             const uint32_t* __restrict__ ctl,
+                                             uint32_t* __restrict__ ctl,
                                              const uint32_t* __restrict__ keys_base,
                                              const uint32_t* __restrict__ vals_base, State src, State dst,
                                              const uint32_t* __restrict__ ids_src, uint32_t* __restrict__ ids_dst,
@@ -691,12 +700,14 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
   const uint32_t sel = sorted_sel(ctl[kCtlMaxKey]);
   const uint32_t* keys = keys_base + (size_t)sel * n;
   const uint32_t* perm = vals_base + (size_t)sel * n;
-  bool first = false;
+  bool first = false, tiny = false;
   uint32_t key = 0u, code = 0u;
   if (s < n) {
     const uint32_t from = min(perm[s], n - 1u);  // in range even after a flagged sort stall
     key = keys[s];
     float4 p = src.pos[from];
+    auto below = [](float x) { return x != 0.f && fabsf(x) < kTinyCoordinate; };
+    tiny = below(p.x) || below(p.y) || below(p.z);
     code = half_code(p, split.morton(key), grids[scene_of[s]]);
     p.w = __uint_as_float(code);
     dst.pos[s] = p;
@@ -720,6 +731,7 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
     if (lane == b) plane = v;
   }
   if (lane < kHalfPlanes && (s & ~31u) < n) planes[(size_t)(s >> 5) * kHalfPlanes + lane] = plane;
+  if (tiny) ctl[kCtlTiny] = 1u;
   const uint32_t bal = __ballot_sync(0xFFFFFFFFu, first);
   if (lane == 0) warp_base[warp] = __popc(bal);
   __syncthreads();
@@ -739,7 +751,7 @@ __device__ __forceinline__ void gather_block(uint32_t vb, uint32_t n, const DevG
 
 static __global__ void __launch_bounds__(kBlock)
     k_gather(uint32_t n, const DevGrid* __restrict__ grids,
-             const uint16_t* __restrict__ scene_of, const uint32_t* __restrict__ ctl,
+             const uint16_t* __restrict__ scene_of, uint32_t* __restrict__ ctl,
              const uint32_t* __restrict__ keys_base,
              const uint32_t* __restrict__ vals_base, State src, State dst,
              const uint32_t* __restrict__ ids_src, uint32_t* __restrict__ ids_dst,
@@ -769,8 +781,6 @@ static __global__ void __launch_bounds__(kBlock)
 // and read with evict-first (streaming) hints: it is read once, and at 1M
 // particles it is larger than L2, where the neighbour records should stay.
 
-constexpr int kGatherBlock = 128;
-
 // Tait pressure (sph.cl:36-39): K * (pown(rho / rho0, 7) - 1).
 __device__ __forceinline__ float tait_pressure(float rho, const Consts& c) {
   const float x = XDIV(rho, c.rho0);
@@ -796,21 +806,23 @@ struct ForceSums {
   float lap;
 };
 
-// One contributing pair of forces.cl:67-97. aux_j = (rho_j, p_j, m/rho_j, p_j/rho_j^2).
-__device__ __forceinline__ void force_pair(ForceSums& f, bool self, V3 d, float rr, float4 vi,
-                                           float4 vj, float4 aux_j, float own, float hh,
-                                           float lap_b, const Consts& c) {
-  const float mj = aux_j.z;
+// One contributing pair of forces.cl:67-97; mj = m/rho_j, qj = p_j/rho_j^2.
+// kShort: the quotients share one reciprocal.
+template <bool kShort>
+__device__ __forceinline__ void force_pair(ForceSums& f, bool self, V3 d, float rr, float4 vi, float4 vj, float mj,
+                                           float qj, float own, float hh, float lap_b, const Consts& c) {
   if (!self) {
-    const float coef = XMUL(XADD(aux_j.w, own), c.mass);
+    const float coef = XMUL(XADD(qj, own), c.mass);
     V3 sg;
     if (XSUB(rr, 0.0000001f) < 0.f) {  // smoothing.cl:23-25
       sg = {c.spiky_zero, c.spiky_zero, c.spiky_zero};
     } else {
       const float q = XSUB(c.h, rr);
       const float q2 = XMUL(q, q);
-      sg = {XMUL(XMUL(c.spiky, XDIV(d.x, rr)), q2), XMUL(XMUL(c.spiky, XDIV(d.y, rr)), q2),
-            XMUL(XMUL(c.spiky, XDIV(d.z, rr)), q2)};
+      const float y = kShort ? rcp_rn_normal(rr) : 0.f;
+      auto over_r = [&](float x) { return kShort ? div_rn_normal(x, rr, y) : XDIV(x, rr); };
+      sg = {XMUL(XMUL(c.spiky, over_r(d.x)), q2), XMUL(XMUL(c.spiky, over_r(d.y)), q2),
+            XMUL(XMUL(c.spiky, over_r(d.z)), q2)};
     }
     f.P.x = XADD(f.P.x, XMUL(coef, sg.x));
     f.P.y = XADD(f.P.y, XMUL(coef, sg.y));
@@ -1143,8 +1155,8 @@ static __global__ void __launch_bounds__(kParticleWarps * 32)
 // serve are done by a whole warp each (density_particle_warp): those on a
 // mid-plane of the cell, so in two octants; cells of up to kSparseCell
 // particles, for which the lists cost more than they save; lists longer than
-// the team's shared memory; and neighbours of a cell of 2048 or more
-// particles, which tags can't address.
+// the team's shared memory; neighbours of a cell of 2048 or more particles,
+// which tags can't address; and scenes whose h is outside near_norm's range.
 //
 // Bound: instruction issue, half of it the exact evaluation. 1,048,576
 // particles spread over a floor (29,552 cells, a quarter of them of one or
@@ -1304,7 +1316,8 @@ __device__ __forceinline__ void density_cells_team(
       const uint32_t own_e = __shfl_sync(0xFFFFFFFFu, e, 13);
       const uint32_t count = own_e > own.x ? own_e - own.x : 0u;
       uint32_t candidates = kNoLists;
-      if (!__any_sync(0xFFFFFFFFu, e - s >= (1u << kCellOffBits)) && count > kSparseCell) {
+      const uint32_t sc = split.shift >= 32u ? 0u : own.y >> split.shift;
+      if (!__any_sync(0xFFFFFFFFu, e - s >= (1u << kCellOffBits)) && count > kSparseCell && consts[sc].plain_h) {
         // the candidates of list k as bits, in up to three words of the planes (more are counted and read again)
         const uint32_t need = kOffsetMasks.m[min(lane, 26u)];
         const uint32_t w0 = s >> 5, words = e > s && lane != 13u ? ((e - 1u) >> 5) - w0 + 1u : 0u;
@@ -1374,7 +1387,6 @@ __device__ __forceinline__ void density_cells_team(
       }
       cell.slot_of[lane] = s - (lane << kCellOffBits);
       if (lane == 0) {
-        const uint32_t sc = split.shift >= 32u ? 0u : own.y >> split.shift;
         const DevGrid& g = grids[sc];
         cell.origin = make_float4(g.lo[0] + ((float)compact_bits3(key) + 0.5f) * g.cell,
                                   g.lo[1] + ((float)compact_bits3(key >> 1) + 0.5f) * g.cell,
@@ -1486,11 +1498,10 @@ __device__ __forceinline__ void density_cells_team(
         float4 pn = pj;
         if (++k < found) pn = next(tagn);
         const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
-        const float rr = xnorm(d);
+        const float rr = near_norm(d);
         if (rr < c.h) {
           rho = XADD(rho, poly6_term(rr, hh, c));
-          if (kept < nlist_cap) __stcs(list, (uint16_t)tag);
-          list += n;
+          if (kept < nlist_cap) __stcs(list + (uint64_t)kept * n, (uint16_t)tag);
           ++kept;
         }
         tag = tagn;
@@ -1524,46 +1535,127 @@ __global__ void __launch_bounds__(Team::kWarps * 32, BLOCKS)
 // Per-pair hook of k_forces (the learned stepper gathers its neighbour
 // features in the same walk); the plain substep uses this empty one.
 struct NoForceHook {
+  static constexpr bool kPairs = false;  // needs no visit of every pair by the particle's own lane
   struct Acc {};
   __device__ __forceinline__ Acc begin(uint32_t) const { return {}; }
   __device__ __forceinline__ void pair(Acc&, uint32_t, uint32_t, const V3&, const V3&) const {}
   __device__ __forceinline__ void end(Acc&, uint32_t, const float4&) const {}
 };
 
+// Forces of one particle by a whole warp, for particles without a complete
+// neighbour list: the window's cells in the reference's order, 32 candidates
+// at a time; each lane evaluates its candidate and the contributing terms are
+// added one after another in lane order, which is the reference's sequence.
+// (One lane alone walks its 500 to 1,000 candidates in about 150 us, which a
+// single such particle adds to the kernel; the warp takes a few us.)
+__device__ __forceinline__ void forces_particle_warp(uint32_t i, uint32_t n, const DevGrid* grids,
+                                                     const uint16_t* scene_of, const uint32_t* ctl,
+                                                     const uint32_t* keys_base, const State& st, const float4* aux,
+                                                     const CellIndex& ci, const Consts* consts, float4* acc_out,
+                                                     const float4* frec) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t sc = scene_of[i];
+  const Consts& c = consts[sc];
+  const KeySplit split{ctl[kCtlShift]};
+  const float4 pi = st.pos[i], vi = st.vel[i], ai = aux[i];
+  const float hh = XMUL(c.h, c.h), lap_b = XMUL(3.f, hh);
+  const Window w = neighbour_window(pi, split.morton(keys_base[(size_t)sorted_sel(ctl[kCtlMaxKey]) * n + i]), grids[sc]);
+  ForceSums f = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, 0.f};
+  for (uint32_t z = w.lo[2]; z <= w.hi[2]; ++z)
+    for (uint32_t y = w.lo[1]; y <= w.hi[1]; ++y)
+      for (uint32_t x = w.lo[0]; x <= w.hi[0]; ++x) {
+        const uint2 r = cell_lookup(ci, morton3(x, y, z) | split.scene_bits(sc));
+        for (uint32_t base = r.x; base < r.y; base += 32u) {
+          const uint32_t j = base + lane;
+          bool hit = false;
+          ForceSums t{};
+          if (j < r.y) {
+            const float4 pj = frec[j];
+            const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
+            const float rr = xnorm(d);
+            hit = near_cull(pi, pj, c.cull_r2) && rr < c.h;
+            if (hit) {
+              const float4 vj = frec[(size_t)n + j];
+              force_pair<false>(t, j == i, d, rr, vi, vj, pj.w, vj.w, ai.w, hh, lap_b, c);
+            }
+          }
+          for (uint32_t bal = __ballot_sync(0xFFFFFFFFu, hit); bal; bal &= bal - 1u) {
+            const int l = __ffs(bal) - 1;
+            // (a sum that starts at +0 is never -0, so adding the +0 of a term that doesn't count changes nothing)
+            auto add = [&](float& sum, float term) { sum = XADD(sum, __shfl_sync(0xFFFFFFFFu, term, l)); };
+            auto add3 = [&](V3& sum, const V3& term) { add(sum.x, term.x), add(sum.y, term.y), add(sum.z, term.z); };
+            add3(f.P, t.P), add3(f.Vs, t.Vs), add3(f.Nm, t.Nm), add(f.lap, t.lap);
+          }
+        }
+      }
+  if (lane == 0) acc_out[i] = finish_accel(f, ai.x, c);
+}
+
+// The same by the particle's own lane, for hooks that visit every pair.
+template <class Hook>
+__device__ __forceinline__ void forces_particle_alone(uint32_t i, uint32_t n, const DevGrid* grids,
+                                                      const uint16_t* scene_of, const uint32_t* ctl,
+                                                      const uint32_t* keys_base, const State& st, const float4* aux,
+                                                      const CellIndex& ci, const Consts* consts, float4* acc_out,
+                                                      const Hook& hook, const float4* frec) {
+  typename Hook::Acc ha = hook.begin(i);
+  const uint32_t sc = scene_of[i];
+  const Consts& c = consts[sc];
+  const KeySplit split{ctl[kCtlShift]};
+  const float4 pi = st.pos[i], vi = st.vel[i], ai = aux[i];
+  const float hh = XMUL(c.h, c.h), lap_b = XMUL(3.f, hh);
+  const Window w = neighbour_window(pi, split.morton(keys_base[(size_t)sorted_sel(ctl[kCtlMaxKey]) * n + i]), grids[sc]);
+  ForceSums f = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, 0.f};
+  for_each_candidate(w, split.scene_bits(sc), ci, [&](uint32_t j) {
+    const float4 pj = frec[j];
+    if (!near_cull(pi, pj, c.cull_r2)) return;
+    const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
+    const float rr = xnorm(d);
+    if (!(rr < c.h)) return;
+    const float4 vj = frec[(size_t)n + j];
+    force_pair<false>(f, j == i, d, rr, vi, vj, pj.w, vj.w, ai.w, hh, lap_b, c);
+    hook.pair(ha, i, j, d, V3{XSUB(vj.x, vi.x), XSUB(vj.y, vi.y), XSUB(vj.z, vi.z)});
+  });
+  const float4 a = finish_accel(f, ai.x, c);
+  acc_out[i] = a;
+  hook.end(ha, i, a);
+}
+
 // Internal forces (forces.cl:45-112) -> acceleration (sph.cl:53-58), walking
-// the neighbour list of k_density (or the window, for overflowing lists).
+// the neighbour list of the density kernel (or the window, for particles
+// without a complete list and scenes outside the short quotients' range).
+// Whole warps call it; `valid`: the lane has a particle.
+//
+// Bound: latency of the record gathers and FP32 issue. The quotients of a pair
+// share one reciprocal and the square root has no slow path: 64 registers, 32
+// warps an SM, instead of 72 and 28; 1,048,576 particles (25 neighbours on
+// average) 0.186 -> 0.155 ms, with the learned step's features 0.361 -> 0.256
+// (at most 102 registers: the features' 22 sums; unbounded, the compiler took
+// 113 and 0.310 ms).
 template <class Hook>
 __device__ __forceinline__ void forces_particle(
-    uint32_t i, uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
-    const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ keys_base, State st,
-    const float4* __restrict__ aux, CellIndex ci, const Consts* __restrict__ consts,
+    bool valid, uint32_t i, uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
+    const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ keys_base, const State& st,
+    const float4* __restrict__ aux, const CellIndex& ci, const Consts* __restrict__ consts,
     const uint16_t* __restrict__ nlist, const uint32_t* __restrict__ ncount, uint32_t nlist_cap,
     float4* __restrict__ acc_out, const Hook& hook, const float4* __restrict__ frec,
     const uint32_t* __restrict__ nb_start) {
-  typename Hook::Acc ha = hook.begin(i);
-  const uint32_t sc = scene_of[i];
-  const Consts c = consts[sc];
+  if (!valid) i = 0;
+  // (every load of the prologue is issued before the first is used)
+  auto tag_at = [&](uint32_t k) { return (uint32_t)__ldcs(&nlist[(size_t)k * n + i]); };
+  const uint32_t t0 = tag_at(0), t1 = tag_at(1), t2 = tag_at(2);
+  const uint32_t cnt = ncount[i];
   const float4 pi = st.pos[i];
   const float4 vi = st.vel[i];
   const float4 ai = aux[i];
-  const float own = ai.w;
-  const float hh = XMUL(c.h, c.h);
-  const float lap_b = XMUL(3.f, hh);
-  ForceSums f = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, 0.f};
-  // neighbour data from the density kernel's 32-byte records
-  auto pair_with = [&](uint32_t j, const float4& pj, const float4& sj) {
-    const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
-    const float rr = xnorm(d);
-    const float4 vj = make_float4(sj.x, sj.y, sj.z, 0.f);
-    force_pair(f, j == i, d, rr, vi, vj, make_float4(0.f, 0.f, pj.w, sj.w), own, hh, lap_b, c);
-    // the same differences force_pair forms (the compiler shares them); dead
-    // code for the plain substep's empty hook
-    const V3 dv = {XSUB(vj.x, vi.x), XSUB(vj.y, vi.y), XSUB(vj.z, vi.z)};
-    hook.pair(ha, i, j, d, dv);
-  };
-  auto pair = [&](uint32_t j) { pair_with(j, __ldg(&frec[j]), __ldg(&frec[(size_t)n + j])); };
-  const uint32_t cnt = ncount[i];
-  if (cnt <= nlist_cap) {
+  const Consts c = consts[scene_of[i]];
+  const bool listed = valid && cnt <= nlist_cap && c.plain_h && !ctl[kCtlTiny];
+  if (listed) {
+    typename Hook::Acc ha = hook.begin(i);
+    const float own = ai.w;
+    const float hh = XMUL(c.h, c.h);
+    const float lap_b = XMUL(3.f, hh);
+    ForceSums f = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, 0.f};
     // a tag names the neighbour's cell among the 27 around the own cell and
     // its offset there; the own cell's nb_start row holds their first slots
     const uint32_t* nbs = nb_start + (size_t)__float_as_uint(ai.z) * 27u;
@@ -1572,46 +1664,44 @@ __device__ __forceinline__ void forces_particle(
     };
     // software pipeline: while a pair is evaluated, the tag three pairs
     // ahead is loaded, the tag two ahead is resolved to its slot and the
-    // records of the next pair are loaded
+    // records of the next pair (the density kernel's 32 bytes) are loaded
     if (cnt > 0) {
-      auto tag_at = [&](uint32_t k) { return (uint32_t)__ldcs(&nlist[(size_t)k * n + i]); };
-      const uint32_t t0 = tag_at(0);
-      const uint32_t t1 = cnt > 1 ? tag_at(1) : t0;
-      uint32_t tnn = cnt > 2 ? tag_at(2) : t1;
+      uint32_t tnn = cnt > 2 ? t2 : cnt > 1 ? t1 : t0;
       uint32_t j = slot(t0);
-      uint32_t jn = slot(t1);
-      float4 pj = __ldg(&frec[j]), sj = __ldg(&frec[(size_t)n + j]);
+      uint32_t jn = slot(cnt > 1 ? t1 : t0);
+      float4 pj = __ldg(&frec[j]), vj = __ldg(&frec[(size_t)n + j]);
       for (uint32_t k = 0; k < cnt; ++k) {
         const uint32_t t3 = k + 3 < cnt ? tag_at(k + 3) : tnn;
         const uint32_t jnn = slot(tnn);
-        const float4 pn = __ldg(&frec[jn]), sn = __ldg(&frec[(size_t)n + jn]);
-        pair_with(j, pj, sj);
+        const float4 pn = __ldg(&frec[jn]), vn = __ldg(&frec[(size_t)n + jn]);
+        const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
+        force_pair<true>(f, j == i, d, near_norm(d), vi, vj, pj.w, vj.w, own, hh, lap_b, c);
+        // the same differences the terms use (the compiler shares them); dead
+        // code for the plain substep's empty hook
+        const V3 dv = {XSUB(vj.x, vi.x), XSUB(vj.y, vi.y), XSUB(vj.z, vi.z)};
+        hook.pair(ha, i, j, d, dv);
         j = jn;
         jn = jnn;
         pj = pn;
-        sj = sn;
+        vj = vn;
         tnn = t3;
       }
     }
-  } else {
-    const KeySplit split{ctl[kCtlShift]};
-    const uint32_t* keys = keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n;
-    const Window w = neighbour_window(pi, split.morton(keys[i]), grids[sc]);
-    for_each_candidate(w, split.scene_bits(sc), ci, [&](uint32_t j) {
-      const float4 pj = __ldg(&frec[j]);
-      const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-      if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > c.cull_r2) return;
-      const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
-      if (xnorm(d) < c.h) pair(j);
-    });
+    const float4 a = finish_accel(f, ai.x, c);
+    acc_out[i] = a;
+    hook.end(ha, i, a);
   }
-  const float4 a = finish_accel(f, ai.x, c);
-  acc_out[i] = a;
-  hook.end(ha, i, a);
+  if constexpr (!Hook::kPairs) {
+    for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, valid && !listed); rest; rest &= rest - 1u)
+      forces_particle_warp(__shfl_sync(0xFFFFFFFFu, i, __ffs(rest) - 1), n, grids, scene_of, ctl, keys_base, st, aux,
+                           ci, consts, acc_out, frec);
+  } else if (valid && !listed) {
+    forces_particle_alone(i, n, grids, scene_of, ctl, keys_base, st, aux, ci, consts, acc_out, hook, frec);
+  }
 }
 
 template <int BLOCK, class Hook = NoForceHook>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, Hook::kPairs ? 640 / BLOCK : 1024 / BLOCK)
     k_forces(uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
              const uint32_t* __restrict__ ctl,
              const uint32_t* __restrict__ keys_base, State st, const float4* __restrict__ aux,
@@ -1620,8 +1710,8 @@ __global__ void __launch_bounds__(BLOCK)
              float4* __restrict__ acc_out, Hook hook, const float4* __restrict__ frec,
              const uint32_t* __restrict__ nb_start) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  forces_particle(i, n, grids, scene_of, ctl, keys_base, st, aux, ci, consts, nlist, ncount, nlist_cap,
+  if ((i & ~31u) >= n) return;  // whole warps
+  forces_particle(i < n, i, n, grids, scene_of, ctl, keys_base, st, aux, ci, consts, nlist, ncount, nlist_cap,
                   acc_out, hook, frec, nb_start);
 }
 

@@ -50,6 +50,7 @@ constexpr uint32_t kSplitK = 1024;    // batch rows per split of the weight-grad
 enum FeatureMode { kFeatStd = 0, kFeatRaw = 1, kFeatRing = 2 };
 
 struct FeatureHook {
+  static constexpr bool kPairs = true;
   State st;  // sorted state of the current substep
   const float4* aux;
   const Consts* consts;

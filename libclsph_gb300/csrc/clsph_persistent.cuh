@@ -152,8 +152,8 @@ static __global__ void __launch_bounds__(kPersistThreads, 3)
                        blockIdx.x * (kPersistThreads / 64u) + (threadIdx.x >> 6), gridDim.x * (kPersistThreads / 64u),
                        1u + (threadIdx.x >> 6));
     if (!grid_barrier(a, ok_s)) return;
-    for (uint32_t i = gtid; i < n; i += gstride)
-      forces_particle(i, n, a.grids, a.scene_of, a.ctl, a.keys, a.st[1], a.aux, a.ci, a.consts, a.nlist, a.ncount,
+    for (uint32_t i = gtid; (i & ~31u) < n; i += gstride)
+      forces_particle(i < n, i, n, a.grids, a.scene_of, a.ctl, a.keys, a.st[1], a.aux, a.ci, a.consts, a.nlist, a.ncount,
                       a.nlist_cap, a.acc, NoForceHook{}, a.frec, a.nb_start);
     if (!grid_barrier(a, ok_s)) return;
     advect_blocks<false>(blockIdx.x, gridDim.x, n, a.st[1], a.acc, a.st[0], a.meshes, a.consts, a.scene_of,
