@@ -82,8 +82,8 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
   return c;
 }
 
-// Density search of a new handle (clsph_gpu_set_neighbour_search,
-// clsph_gpu_set_launch_shape and clsph_gpu_autotune replace it). Measured
+// Launch shapes of a new handle (clsph_gpu_set_neighbour_search,
+// clsph_gpu_set_launch_shape and clsph_gpu_autotune replace them). Measured
 // (density kernel, us; one warp per particle / teams of 4 / of 2 warps):
 //   water, spread on a floor: 4,096 particles 16 / 27 / 34; 10,000 23 / 29 / 38;
 //   20,000 37 / 34 / 42; 32,768 55 / 35 / 44; 65,536 102 / 53 / 52;
@@ -95,11 +95,15 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
 // particles at rest (38 at 20 particles within the radius, 76 at 40) also take
 // the larger lists: shared memory for 92 chunks lets 16 teams of two share an
 // SM, for 128 chunks 12 (1,048,576 particles of water: 0.309 against 0.346 ms).
-void choose_search(clsph_gpu* h) {
+void choose_shapes(clsph_gpu* h) {
   for (const Consts& c : h->consts_host)
     if (!(8.f * c.h * c.h * c.h * c.rho0 <= 50.f * c.mass)) h->packed_cells = true;
   h->search = h->n <= 14000u ? CLSPH_SEARCH_PARTICLE_WARPS : CLSPH_SEARCH_CELL_WARPS;
   h->density_block = h->packed_cells || h->n <= 64000u ? 128 : 64;
+  // advection blocks per SM: blocks of 1,000 to 2,000 consecutive particles even out their collisions
+  // (4,194,304 particles on a heightfield: 8 / 16 / 32 / 64 blocks 0.329 / 0.295 / 0.289 / 0.311 ms; 1,048,576
+  // on a floor: 8 / 16 0.038 / 0.041)
+  h->advect_blocks_per_sm = h->n > 2000000u ? 16u : 8u;
 }
 
 }  // namespace
@@ -481,7 +485,7 @@ int clsph_gpu_create_batched(const clsph_parameters* params, const clsph_kernel_
       return bail(rc);
   }
   h->ntiles = (n + kRadixTile - 1) / kRadixTile;
-  choose_search(h);
+  choose_shapes(h);
   uint32_t slots = 1024;
   while (slots < 2u * n) slots <<= 1;
   h->slots = slots;
@@ -610,14 +614,16 @@ int clsph_gpu_set_scene_mesh(clsph_gpu* h, uint32_t scene, const float* normals,
     int rc;
     if ((rc = dev_alloc(&sm.normals, 3 * (size_t)faces)) ||
         (rc = dev_alloc(&sm.vertices, 3 * (size_t)vertex_count)) ||
-        (rc = dev_alloc(&sm.indices, 3 * (size_t)faces)))
+        (rc = dev_alloc(&sm.indices, 3 * (size_t)faces)) ||
+        (rc = dev_alloc(&sm.packed, kFaceRows * (size_t)faces)))
       return rc;
     CUDA_TRY(cudaMemcpy(sm.normals, normals, sizeof(float) * 3 * faces, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(sm.vertices, vertices, sizeof(float) * 3 * vertex_count, cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(sm.indices, indices, sizeof(uint32_t) * 3 * faces, cudaMemcpyHostToDevice));
-    dm.normals = sm.normals;
-    dm.vertices = sm.vertices;
-    dm.indices = sm.indices;
+    k_pack_faces<<<grid_blocks(faces, h->sm_count * 8), kBlock, 0, h->stream>>>(sm.normals, sm.vertices, sm.indices,
+                                                                                faces, sm.packed);
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    dm.packed = sm.packed;
     dm.faces = faces;
     FaceGridPlan plan{};
     float reach = 0.f;

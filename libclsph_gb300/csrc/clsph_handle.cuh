@@ -80,6 +80,7 @@ struct SceneMesh {
   float* normals = nullptr;
   float* vertices = nullptr;
   uint32_t* indices = nullptr;
+  float4* packed = nullptr;  // the collision test's rows
   uint32_t* cell_start = nullptr;
   uint32_t* cell_faces = nullptr;
   FaceGridPlan plan{};    // grid of the per-cell triangle lists
@@ -88,6 +89,7 @@ struct SceneMesh {
     cudaFree(normals);
     cudaFree(vertices);
     cudaFree(indices);
+    cudaFree(packed);
     cudaFree(cell_start);
     cudaFree(cell_faces);
     *this = SceneMesh{};

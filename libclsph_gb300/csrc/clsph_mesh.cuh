@@ -106,6 +106,27 @@ static __global__ void k_face_fill(const float* __restrict__ vx, const uint32_t*
               [&](uint32_t f, uint32_t c) { list[start[c] + atomicAdd(&fill[c], 1u)] = f; });
 }
 
+// What the collision test reads of a face, in kFaceRows rows of 16 bytes:
+// normal and its length; v0 and u.v; u = v1 - v0 and u.u; v = v2 - v0 and v.v
+// (collisions.cl:21-60 forms these per particle and face; the operations and
+// their order are the same).
+constexpr uint32_t kFaceRows = 4;
+static __global__ void k_pack_faces(const float* __restrict__ normals, const float* __restrict__ vx,
+                                    const uint32_t* __restrict__ ix, uint32_t faces, float4* __restrict__ out) {
+  for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f < faces; f += gridDim.x * blockDim.x) {
+    auto vertex = [&](uint32_t k) {
+      const float* p = vx + 3 * (size_t)ix[3 * f + k];
+      return V3{p[0], p[1], p[2]};
+    };
+    const V3 nrm = {normals[3 * f], normals[3 * f + 1], normals[3 * f + 2]};
+    const V3 v0 = vertex(0), u = xsub3(vertex(1), v0), v = xsub3(vertex(2), v0);
+    out[kFaceRows * (size_t)f] = make_float4(nrm.x, nrm.y, nrm.z, xnorm(nrm));
+    out[kFaceRows * (size_t)f + 1] = make_float4(v0.x, v0.y, v0.z, xdot(u, v));
+    out[kFaceRows * (size_t)f + 2] = make_float4(u.x, u.y, u.z, xdot(u, u));
+    out[kFaceRows * (size_t)f + 3] = make_float4(v.x, v.y, v.z, xdot(v, v));
+  }
+}
+
 static __global__ void k_face_sort(const uint32_t* __restrict__ start, uint32_t cells, uint32_t* __restrict__ list) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
     const uint32_t b = start[c], e = start[c + 1];
