@@ -390,7 +390,7 @@ int gemm_tc(cudaStream_t s, uint32_t* err, const bf16* A, int lda, const bf16* B
             int k_split, Epi epi) {
   using L = clsph_nn::GemmTcLayout<BN>;
   (void)sizeof(L);
-  if (N != BN || M % clsph_nn::kGtRows || k_split <= 0 || K % k_split || k_split % clsph_nn::kGtBK ||
+  if (N != BN || M % clsph_nn::kGtRows || k_split <= 0 || K % k_split || k_split % 32 ||
       lda % 8 || ldb % 8)
     return fail(CLSPH_ERR_ARGUMENT, "mlp: GEMM shape not tileable");
   auto kernel = clsph_nn::k_gemm_tc<BN, A_K, B_K, Epi>;
@@ -477,28 +477,27 @@ int pass(clsph_mlp* m, uint32_t rows, float* loss_slot, bool backward) {
   int rc;
   if (backward) CUDA_TRY(cudaMemsetAsync(m->grad, 0, sizeof(float) * kParams, s));
   uint32_t* err = m->err;
-  // Z1 = X W1 + b1, H1 = GELU(Z1)
-  if ((rc = gemm_tc<kHid, true, false>(s, err, m->xb, kIn, m->w1b, kHid, rows, kHid, kIn, kIn,
-                                       EpiHidden{p + clsph_nn::kOffB1, m->z1, m->h1, kHid})))
+  // Z1 = X W1 + b1, H1 = GELU(Z1); the weights with K contiguous, so that both operands are copied as they lie
+  if ((rc = gemm_tc<kHid, true, true>(s, err, m->xb, kIn, m->w1t, kIn, rows, kHid, kIn, kIn,
+                                      EpiHidden{p + clsph_nn::kOffB1, m->z1, m->h1, kHid, 1.f})))
     return rc;
-  // Z2 = H1 W2 + b2, H2 = GELU(Z2)
-  if ((rc = gemm_tc<kHid, true, false>(s, err, m->h1, kHid, m->w2b, kHid, rows, kHid, kHid, kHid,
-                                       EpiHidden{p + clsph_nn::kOffB2, m->z2, m->h2, kHid})))
+  // Z2 = H1 W2 + b2, H2 = GELU(Z2) (w2t holds W2 / 2)
+  if ((rc = gemm_tc<kHid, true, true>(s, err, m->h1, kHid, m->w2t, kHid, rows, kHid, kHid, kHid,
+                                      EpiHidden{p + clsph_nn::kOffB2, m->z2, m->h2, kHid, 2.f})))
     return rc;
-  // Y = H2 W3 + b3, loss, dZ2, dW3, db3
-  clsph_nn::k_head<<<rows / 256, kHid, 0, s>>>(m->h2, m->z2, p + clsph_nn::kOffW3, p + clsph_nn::kOffB3, m->yb,
-                                               rows, 256, 1.f / rows, m->dz2, m->grad + clsph_nn::kOffW3,
-                                               m->grad + clsph_nn::kOffB3, loss_slot, nullptr);
+  // Y = H2 W3 + b3, loss, dZ2, dW3, db3, db2
+  clsph_nn::k_head<<<std::min(rows / clsph_nn::kHeadWarps, 2 * m->sms), clsph_nn::kHeadWarps * 32, 0, s>>>(
+      m->h2, m->z2, p + clsph_nn::kOffW3, p + clsph_nn::kOffB3, m->yb, rows, 1.f / rows, m->dz2,
+      m->grad + clsph_nn::kOffW3, m->grad + clsph_nn::kOffB3, m->grad + clsph_nn::kOffB2, loss_slot);
   if (!backward) return 0;
   const int splits = rows / kSplitK;
   const size_t split_stride = (size_t)kHid * kHid;
-  // dW2 = H1^T dZ2 (split over rows), db2 = column sums of dZ2
+  // dW2 = H1^T dZ2 (split over rows)
   if ((rc = gemm_tc<kHid, false, false>(s, err, m->h1, kHid, m->dz2, kHid, kHid, kHid, rows, kSplitK,
                                         EpiPartial{m->ws, kHid, split_stride})))
     return rc;
   clsph_nn::k_reduce_splits<<<(kHid * kHid + 255) / 256, 256, 0, s>>>(m->ws, splits, (size_t)kHid * kHid,
                                                                       m->grad + clsph_nn::kOffW2);
-  clsph_nn::k_colsum<<<rows / 256, kHid, 0, s>>>(m->dz2, rows, kHid, 256, m->grad + clsph_nn::kOffB2);
   // dZ1 = (dZ2 W2^T) * GELU'(Z1)
   if ((rc = gemm_tc<kHid, true, true>(s, err, m->dz2, kHid, m->w2b, kHid, rows, kHid, kHid, kHid,
                                       EpiGeluGrad{m->z1, m->dz1, kHid})))
@@ -510,7 +509,7 @@ int pass(clsph_mlp* m, uint32_t rows, float* loss_slot, bool backward) {
     return rc;
   clsph_nn::k_reduce_splits<<<(kIn * kHid + 255) / 256, 256, 0, s>>>(m->ws, splits, (size_t)kIn * kHid,
                                                                     m->grad + clsph_nn::kOffW1);
-  clsph_nn::k_colsum<<<rows / 256, kHid, 0, s>>>(m->dz1, rows, kHid, 256, m->grad + clsph_nn::kOffB1);
+  clsph_nn::k_colsum<<<rows / 256, kHid, 0, s>>>(m->dz1, rows, 256, m->grad + clsph_nn::kOffB1);
   return 0;
 }
 
@@ -905,13 +904,10 @@ int clsph_mlp_gradients(clsph_mlp* m, const float* x_raw, const float* y_raw, ui
   if (!m || !x_raw || !y_raw || rows == 0 || rows % kRowBlock)
     return fail(CLSPH_ERR_ARGUMENT, "mlp_gradients: rows must be a positive multiple of 2048");
   int rc;
-  if ((rc = ensure_training(m, rows)) || (rc = ensure_idx(m, rows)) || (rc = ensure_loss(m, 1))) return rc;
-  std::vector<uint32_t> iota(rows);
-  std::iota(iota.begin(), iota.end(), 0u);
-  CUDA_TRY(cudaMemcpyAsync(m->idx, iota.data(), sizeof(uint32_t) * rows, cudaMemcpyHostToDevice, m->stream));
+  if ((rc = ensure_training(m, rows)) || (rc = ensure_loss(m, 1))) return rc;
   CUDA_TRY(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
   clsph_nn::k_gather_batch<<<(rows * (kIn + kOut) + 255) / 256, 256, 0, m->stream>>>(
-      x_raw, y_raw, m->idx, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
+      x_raw, y_raw, nullptr, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
   if ((rc = pass(m, rows, m->loss, true))) return rc;
   float l = 0.f;
   CUDA_TRY(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -929,19 +925,16 @@ int clsph_mlp_loss(clsph_mlp* m, const float* x_raw, const float* y_raw, uint64_
   if (rows == 0) return fail(CLSPH_ERR_ARGUMENT, "mlp_loss: fewer than 2048 samples");
   const uint64_t blocks = samples / rows;
   int rc;
-  if ((rc = ensure_training(m, rows)) || (rc = ensure_idx(m, rows)) || (rc = ensure_loss(m, 1))) return rc;
+  if ((rc = ensure_training(m, rows)) || (rc = ensure_loss(m, 1))) return rc;
   CUDA_TRY(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-  std::vector<uint32_t> iota(rows);
   for (uint64_t b = 0; b < blocks; ++b) {
-    for (uint32_t r = 0; r < rows; ++r) iota[r] = (uint32_t)(b * rows + r);
-    CUDA_TRY(cudaMemcpyAsync(m->idx, iota.data(), sizeof(uint32_t) * rows, cudaMemcpyHostToDevice, m->stream));
     clsph_nn::k_gather_batch<<<(rows * (kIn + kOut) + 255) / 256, 256, 0, m->stream>>>(
-        x_raw, y_raw, m->idx, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
+        x_raw + b * rows * kIn, y_raw + b * rows * kOut, nullptr, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
     if ((rc = pass(m, rows, m->loss, false))) return rc;
-    CUDA_TRY(cudaStreamSynchronize(m->stream));  // iota is reused
   }
   float l = 0.f;
-  CUDA_TRY(cudaMemcpy(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+  CUDA_TRY(cudaStreamSynchronize(m->stream));
   if ((rc = check_train_waits(m))) return rc;
   *loss = l / (float)(blocks * rows);
   return CLSPH_OK;

@@ -325,14 +325,17 @@ __global__ void __launch_bounds__(kInferWarps * 32, 1)
 // Epilogue functors of the training GEMM (k_gemm_tc in clsph_mlp_tc.cuh),
 // called on every (row, even column) pair of the product.
 
-// z = acc + bias; Z (fp32) and H = GELU(z) (bf16), both [M][ld]
+// z = scale acc + bias (scale a power of two); Z (fp32) and H = GELU(z) (bf16), both [M][ld]
 struct EpiHidden {
+  static constexpr bool kByRow = false;  // lanes take columns of a row, so that rows are written whole
   const float* bias;
   float* z;
   bf16* h;
   int ld;
+  float scale;
   __device__ void operator()(int row, int col, float v0, float v1) const {
-    const float z0 = v0 + bias[col], z1 = v1 + bias[col + 1];
+    const float2 b = __ldg(reinterpret_cast<const float2*>(bias + col));
+    const float z0 = fmaf(v0, scale, b.x), z1 = fmaf(v1, scale, b.y);
     const size_t o = (size_t)row * ld + col;
     *reinterpret_cast<float2*>(z + o) = make_float2(z0, z1);
     *reinterpret_cast<uint32_t*>(h + o) = GeluConsts()(z0, z1);
@@ -341,18 +344,20 @@ struct EpiHidden {
 
 // dZ = acc * GELU'(Z), stored bf16 [M][ld]
 struct EpiGeluGrad {
+  static constexpr bool kByRow = false;
   const float* z;
   bf16* dz;
   int ld;
   __device__ void operator()(int row, int col, float v0, float v1) const {
     const size_t o = (size_t)row * ld + col;
-    const float2 zz = *reinterpret_cast<const float2*>(z + o);
+    const float2 zz = __ldg(reinterpret_cast<const float2*>(z + o));
     *reinterpret_cast<uint32_t*>(dz + o) = pack_bf16(v0 * gelu_grad(zz.x), v1 * gelu_grad(zz.y));
   }
 };
 
 // split-K partial sums, ws[blockIdx.z][M][ld]
 struct EpiPartial {
+  static constexpr bool kByRow = false;
   float* ws;
   int ld;
   size_t split_stride;
@@ -365,6 +370,7 @@ struct EpiPartial {
 // split-K partial sums of a transposed product: the GEMM computes C^T, so
 // element (row, col) of it is C's (col, row), ws[blockIdx.z][col][ld]
 struct EpiPartialT {
+  static constexpr bool kByRow = true;  // a lane's row is a column of C: consecutive lanes write consecutive words
   float* ws;
   int ld;
   size_t split_stride;
@@ -380,13 +386,13 @@ struct EpiPartialT {
 
 // Batch rows from the sample set: x standardised to bf16, y standardised fp32.
 __global__ void k_gather_batch(const float* __restrict__ x_raw, const float* __restrict__ y_raw,
-                               const uint32_t* __restrict__ idx, uint32_t rows,
+                               const uint32_t* __restrict__ idx /* or null: the rows as they lie */, uint32_t rows,
                                const float* __restrict__ norm /* blob + kOffXMu */,
                                bf16* __restrict__ xb, float* __restrict__ yb) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t r = t / (kIn + kOut), c = t % (kIn + kOut);
   if (r >= rows) return;
-  const size_t s = idx[r];
+  const size_t s = idx ? idx[r] : r;
   if (c < kIn) {
     const float v = standardise(x_raw[s * kIn + c], norm[c], norm[kIn + c]);
     xb[(size_t)r * kIn + c] = __float2bfloat16_rn(v);
@@ -405,77 +411,127 @@ __global__ void k_standardize(const float* __restrict__ x_raw, uint32_t rows, co
   xb[i] = __float2bfloat16_rn(standardise(x_raw[i], norm[c], norm[kIn + c]));
 }
 
-// Layer 3 forward + loss + backward to dZ2, one block of 256 threads (one per
-// hidden unit) walking `rows_per_block` rows:
+// Layer 3 forward + loss + backward to dZ2, one warp per row (lane l: hidden
+// units 8 l .. 8 l + 7), the rows shared out over all blocks' warps:
 //   y = H2 W3 + b3, loss = mean over rows of sum_k (y_k - t_k)^2,
 //   dY = 2 (y - t) / rows, dZ2 = (dY W3^T) * GELU'(Z2),
-//   dW3 += H2^T dY, db3 += sum dY, loss_sum += sum of squared errors.
-__global__ void __launch_bounds__(kHid)
+//   dW3 += H2^T dY, db3 += sum dY, db2 += sum dZ2, loss_sum += sum of squared errors.
+// (One block per row, with three barriers and a lone thread's sum each, took
+// 0.40 ms for 65,536 rows, and the column sums of dZ2 a pass of their own.)
+constexpr int kHeadWarps = 8;
+__global__ void __launch_bounds__(kHeadWarps * 32)
     k_head(const bf16* __restrict__ h2, const float* __restrict__ z2, const float* __restrict__ w3,
-           const float* __restrict__ b3, const float* __restrict__ yt, uint32_t rows,
-           uint32_t rows_per_block, float inv_rows, bf16* __restrict__ dz2, float* __restrict__ dw3,
-           float* __restrict__ db3, float* __restrict__ loss_sum, float* __restrict__ y_out) {
-  __shared__ float red[kHid / 32][kOut];
-  __shared__ float dy_s[kOut];
-  const int k = threadIdx.x, lane = k & 31, warp = k >> 5;
-  float w[kOut];  // BF16 values, as the inference kernels use them
+           const float* __restrict__ b3, const float* __restrict__ yt, uint32_t rows, float inv_rows, bf16* __restrict__ dz2, float* __restrict__ dw3,
+           float* __restrict__ db3, float* __restrict__ db2, float* __restrict__ loss_sum) {
+  static_assert(kHid == 256 && kOut == 4, "eight hidden units a lane");
+  __shared__ float sw[kHid * kOut];
+  __shared__ float sb2[kHid];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float w[8][kOut];  // BF16 values, as the inference kernels use them
 #pragma unroll
-  for (int j = 0; j < kOut; ++j) w[j] = __bfloat162float(__float2bfloat16_rn(w3[k * kOut + j]));
-  float gw[kOut] = {}, gb[kOut] = {}, lsum = 0.f;
-  const uint32_t r_begin = blockIdx.x * rows_per_block;
-  const uint32_t r_end = min(rows, r_begin + rows_per_block);
-  for (uint32_t r = r_begin; r < r_end; ++r) {
-    const size_t o = (size_t)r * kHid + k;
-    const float hv = __bfloat162float(h2[o]);
-    float p[kOut];
+  for (int u = 0; u < 8; ++u) {
+    const float4 q = *reinterpret_cast<const float4*>(w3 + (8 * lane + u) * kOut);
+    const float f[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) w[u][j] = __bfloat162float(__float2bfloat16_rn(f[j]));
+  }
+  const float4 bias = *reinterpret_cast<const float4*>(b3);
+  float gw[8][kOut] = {}, gb2[8] = {}, gb[kOut] = {}, lsum = 0.f;
+  for (uint32_t r = blockIdx.x * kHeadWarps + warp; r < rows; r += gridDim.x * kHeadWarps) {
+    const size_t o = (size_t)r * kHid + 8 * lane;
+    const uint4 hq = *reinterpret_cast<const uint4*>(h2 + o);
+    const float4 za = *reinterpret_cast<const float4*>(z2 + o), zb = *reinterpret_cast<const float4*>(z2 + o + 4);
+    const float4 tq = __ldg(reinterpret_cast<const float4*>(yt + (size_t)r * kOut));
+    const uint32_t hw[4] = {hq.x, hq.y, hq.z, hq.w};
+    float h[8];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      h[2 * u] = __uint_as_float(hw[u] << 16);
+      h[2 * u + 1] = __uint_as_float(hw[u] & 0xFFFF0000u);
+    }
+    float p[kOut] = {};
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) p[j] = fmaf(h[u], w[u][j], p[j]);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) p[j] += __shfl_xor_sync(0xffffffffu, p[j], s);
+    const float e[kOut] = {bias.x + p[0] - tq.x, bias.y + p[1] - tq.y, bias.z + p[2] - tq.z, bias.w + p[3] - tq.w};
+    float d[kOut];
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
-      p[j] = hv * w[j];
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) p[j] += __shfl_xor_sync(0xffffffffu, p[j], s);
+      d[j] = 2.f * e[j] * inv_rows;
+      gb[j] += d[j];
+      lsum += e[j] * e[j];
     }
-    if (lane == 0)
+    const float z[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+    uint32_t out[4];
+    float dz[8];
 #pragma unroll
-      for (int j = 0; j < kOut; ++j) red[warp][j] = p[j];
-    __syncthreads();
-    if (k < kOut) {
-      float y = b3[k];
-      for (int q = 0; q < kHid / 32; ++q) y += red[q][k];
-      const float e = y - yt[(size_t)r * kOut + k];
-      dy_s[k] = 2.f * e * inv_rows;
-      if (y_out) y_out[(size_t)r * kOut + k] = y;
-      lsum += e * e;
-    }
-    __syncthreads();
-    float dh = 0.f;
+    for (int u = 0; u < 8; ++u) {
+      float dh = 0.f;
 #pragma unroll
-    for (int j = 0; j < kOut; ++j) {
-      const float d = dy_s[j];
-      dh += d * w[j];
-      gw[j] += hv * d;
-      gb[j] += d;
+      for (int j = 0; j < kOut; ++j) {
+        dh += d[j] * w[u][j];
+        gw[u][j] += h[u] * d[j];
+      }
+      dz[u] = dh * gelu_grad(z[u]);
     }
-    dz2[o] = __float2bfloat16_rn(dh * gelu_grad(z2[o]));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      out[u] = pack_bf16(dz[2 * u], dz[2 * u + 1]);
+      gb2[2 * u] += __uint_as_float(out[u] << 16);
+      gb2[2 * u + 1] += __uint_as_float(out[u] & 0xFFFF0000u);
+    }
+    *reinterpret_cast<uint4*>(dz2 + o) = make_uint4(out[0], out[1], out[2], out[3]);
+  }
+  for (int q = 0; q < kHeadWarps; ++q) {  // the block's sums, warp after warp
+    if (warp == q)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = 8 * lane + u;
+#pragma unroll
+        for (int j = 0; j < kOut; ++j) sw[k * kOut + j] = gw[u][j] + (q ? sw[k * kOut + j] : 0.f);
+        sb2[k] = gb2[u] + (q ? sb2[k] : 0.f);
+      }
     __syncthreads();
   }
+  for (int i = threadIdx.x; i < kHid * kOut; i += kHeadWarps * 32) atomicAdd(&dw3[i], sw[i]);
+  for (int i = threadIdx.x; i < kHid; i += kHeadWarps * 32) atomicAdd(&db2[i], sb2[i]);
+  if (lane == 0) {  // (every lane holds the same)
 #pragma unroll
-  for (int j = 0; j < kOut; ++j) atomicAdd(&dw3[k * kOut + j], gw[j]);
-  if (k < kOut) {
-    atomicAdd(&db3[k], gb[k]);
+    for (int j = 0; j < kOut; ++j) atomicAdd(&db3[j], gb[j]);
     atomicAdd(loss_sum, lsum);
   }
 }
 
-// db[c] += sum over rows of dz[r][c] (bf16 [rows][cols])
-__global__ void k_colsum(const bf16* __restrict__ dz, uint32_t rows, int cols, uint32_t rows_per_block,
-                         float* __restrict__ db) {
-  const int c = threadIdx.x;
-  if (c >= cols) return;
+// db[c] += sum over rows of dz[r][c] (bf16 [rows][256]): 32 threads a row, eight columns each
+__global__ void __launch_bounds__(256) k_colsum(const bf16* __restrict__ dz, uint32_t rows, uint32_t rows_per_block,
+                                                float* __restrict__ db) {
+  __shared__ float part[8][kHid];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t r_begin = blockIdx.x * rows_per_block;
   const uint32_t r_end = min(rows, r_begin + rows_per_block);
-  float s = 0.f;
-  for (uint32_t r = r_begin; r < r_end; ++r) s += __bfloat162float(dz[(size_t)r * cols + c]);
-  atomicAdd(&db[c], s);
+  float s[8] = {};
+#pragma unroll 4
+  for (uint32_t r = r_begin + warp; r < r_end; r += 8) {
+    const uint4 q = *reinterpret_cast<const uint4*>(dz + (size_t)r * kHid + 8 * lane);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s[2 * u] += __uint_as_float(w[u] << 16);
+      s[2 * u + 1] += __uint_as_float(w[u] & 0xFFFF0000u);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u) part[warp][8 * lane + u] = s[u];
+  __syncthreads();
+  float t = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) t += part[q][threadIdx.x];
+  atomicAdd(&db[threadIdx.x], t);
 }
 
 // out[i] = sum over splits of ws[s][i]

@@ -388,24 +388,32 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 // ---------------------------------------------------------------------------
 // Training GEMM on the tensor cores: C[M x N] = A[M x K] B[K x N] with BF16
-// operands and FP32 accumulation in tensor memory; one CTA of 4 warps per
+// operands and FP32 accumulation in tensor memory; one CTA of 8 warps per
 // 128-row tile of C and all N <= 256 columns, split-K over blockIdx.z, and
 // the epilogue functors of k_gemm on every (row, even column) pair.
 // A_K: A is stored with K contiguous (row m at A + m lda), else with M
 // contiguous (A^T in memory: row k at A + k lda). B_K: B is stored with K
 // contiguous per column n (B + n ldb), else with N contiguous (row k at
-// B + k ldb). Operands are staged 32 K at a time, double-buffered, into the
+// B + k ldb). Operands are staged 64 K at a time, double-buffered, into the
 // canonical no-swizzle K-major core-matrix layout of the inference kernel
-// (element (r, k) at (r / 8) * 512 + (k / 8) * 128 + (r % 8) * 16 +
-// (k % 8) * 2): 16-byte vectors when K is contiguous in memory, else 8
-// two-byte stores per 16-byte vector (the transpose). Thread 0 issues two
-// M128 x N x K16 MMAs per chunk and commits them to the chunk buffer's
-// mbarrier; a buffer is restaged once the MMAs that read it have completed.
-// Every wait is bounded: one that runs out sets *err, the CTA stops issuing,
-// waits (bounded) for its last commit and frees tensor memory.
+// (element (r, k) at (r / 8) * 1024 + (k / 8) * 128 + (r % 8) * 16 +
+// (k % 8) * 2): asynchronous 16-byte copies when K is contiguous in memory,
+// else eight 8-byte loads (four rows, eight K) whose halves are permuted into
+// four 16-byte stores. Thread 0 issues four M128 x N x K16 MMAs per chunk and
+// commits them to the chunk buffer's mbarrier; a buffer is restaged once the
+// MMAs that read it have completed. Every wait is bounded: one that runs out
+// sets *err, the CTA stops issuing, waits (bounded) for its last commit and
+// frees tensor memory. The epilogue turns each warp's 32 x 32 accumulators
+// through shared memory, so that it reads and writes memory by rows.
+//
+// Bound: the FP32 pre-activations and BF16 activations it writes (200 MB per
+// hidden layer of 65,536 rows) and the latency of a tile's phases. One lane
+// per row in the epilogue (eight bytes to a line) and transposes by two-byte
+// stores took 0.30 ms for the hidden layer and 0.27 ms for its weight
+// gradient.
 constexpr int kGtRows = 128;
-constexpr int kGtBK = 32;
-constexpr int kGtThreads = 128;
+constexpr int kGtBK = 64;
+constexpr int kGtThreads = 256;
 constexpr uint32_t kGtSmem = 100 * 1024;  // also keeps two CTAs per SM (512 TMEM columns)
 
 template <int BN>
@@ -420,11 +428,8 @@ struct GemmTcLayout {
   static constexpr uint32_t kCols = BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
   static constexpr uint32_t kIdesc = tc_idesc(kGtRows, BN);
   static_assert(kBytes <= kGtSmem, "shared memory of the tensor-core GEMM");
+  static_assert(BN <= 32 || kGtThreads * 33 * 4 <= kBar, "the epilogue's patches lie in the operand buffers");
 };
-
-__device__ __forceinline__ void st_shared_u16(uint32_t addr, uint16_t v) {
-  asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(addr), "h"(v) : "memory");
-}
 
 // 32 consecutive 32-bit TMEM columns of this thread's lane
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
@@ -443,27 +448,39 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
   for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
 }
 
-// `rows` x 32 K of an operand into the canonical layout at `dst`: K-major in
+// `rows` x 64 K of an operand into the canonical layout at `dst`: K-major in
 // memory (row r at src + r ld, K contiguous) or MN-major (K row k at
-// src + k ld, the rows contiguous)
+// src + k ld, the rows contiguous). `ks` (32 or 64) K are staged.
+constexpr uint32_t kGtGroup = kGtBK / 8 * 128;  // bytes of eight rows
 template <bool KMAJOR>
-__device__ __forceinline__ void gt_stage(uint32_t dst, const bf16* __restrict__ src, int ld, int rows) {
+__device__ __forceinline__ void gt_stage(uint32_t dst, const bf16* __restrict__ src, int ld, int rows, int ks) {
   if constexpr (KMAJOR) {
-    for (int c = threadIdx.x; c < rows * 4; c += kGtThreads) {
-      const int r = c >> 2, q = c & 3;
-      const uint4 v = *reinterpret_cast<const uint4*>(src + (size_t)r * ld + q * 8);
-      st_shared_v4(dst + (r >> 3) * 512 + q * 128 + (r & 7) * 16, v);
+    const int qs = ks / 8, shift = ks == kGtBK ? 3 : 2;
+    for (int c = threadIdx.x; c < rows * qs; c += kGtThreads) {
+      const int r = c >> shift, q = c & (qs - 1);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (r >> 3) * kGtGroup + q * 128 +
+                                                                         (r & 7) * 16),
+                   "l"(src + (size_t)r * ld + q * 8)
+                   : "memory");
     }
   } else {
-    const int vecs = rows / 8;
-    for (int c = threadIdx.x; c < kGtBK * vecs; c += kGtThreads) {
-      const int k = c / vecs, mq = c % vecs;
-      const uint4 v = *reinterpret_cast<const uint4*>(src + (size_t)k * ld + mq * 8);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      const uint32_t base = dst + mq * 512 + (k >> 3) * 128 + (k & 7) * 2;
+    const int quads = rows / 4;
+    for (int c = threadIdx.x; c < ks / 8 * quads; c += kGtThreads) {
+      const int q = c / quads, m = 4 * (c % quads);
+      uint2 v[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
-        st_shared_u16(base + e * 16, (uint16_t)(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xFFFFu));
+      for (int k = 0; k < 8; ++k) v[k] = *reinterpret_cast<const uint2*>(src + (size_t)(8 * q + k) * ld + m);
+      const uint32_t at = dst + (m >> 3) * kGtGroup + q * 128 + (m & 7) * 16;
+      auto pick = [&](uint32_t sel, bool second) {
+        auto w = [&](int k) {
+          return second ? __byte_perm(v[k].y, v[k + 1].y, sel) : __byte_perm(v[k].x, v[k + 1].x, sel);
+        };
+        return make_uint4(w(0), w(2), w(4), w(6));
+      };
+      st_shared_v4(at, pick(0x5410, false));
+      st_shared_v4(at + 16, pick(0x7632, false));
+      st_shared_v4(at + 32, pick(0x5410, true));
+      st_shared_v4(at + 48, pick(0x7632, true));
     }
   }
 }
@@ -479,7 +496,7 @@ __global__ void __launch_bounds__(kGtThreads, 1)
   const int m0 = blockIdx.y * kGtRows;
   const int k_begin = blockIdx.z * k_split;
   const int k_end = min(K, k_begin + k_split);
-  const int chunks = (k_end - k_begin) / kGtBK;
+  const int chunks = (k_end - k_begin + kGtBK - 1) / kGtBK;  // the last may hold 32
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sb + L::kSlot),
                  "r"(L::kCols)
@@ -493,10 +510,12 @@ __global__ void __launch_bounds__(kGtThreads, 1)
   }
   auto stage = [&](int buf, int k0) {
     const uint32_t a = sb + buf * L::kStage, b = a + L::kA;
-    if constexpr (A_K) gt_stage<true>(a, A + (size_t)m0 * lda + k0, lda, kGtRows);
-    else gt_stage<false>(a, A + (size_t)k0 * lda + m0, lda, kGtRows);
-    if constexpr (B_K) gt_stage<true>(b, B + k0, ldb, BN);
-    else gt_stage<false>(b, B + (size_t)k0 * ldb, ldb, BN);
+    const int ks = min(kGtBK, k_end - k0);
+    if constexpr (A_K) gt_stage<true>(a, A + (size_t)m0 * lda + k0, lda, kGtRows, ks);
+    else gt_stage<false>(a, A + (size_t)k0 * lda + m0, lda, kGtRows, ks);
+    if constexpr (B_K) gt_stage<true>(b, B + k0, ldb, BN, ks);
+    else gt_stage<false>(b, B + (size_t)k0 * ldb, ldb, BN, ks);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     fence_async_smem();
   };
   if (chunks > 0) stage(0, k_begin);
@@ -512,9 +531,9 @@ __global__ void __launch_bounds__(kGtThreads, 1)
     if (tid == 0) {
       tc_fence_after();
       const uint32_t a = sb + buf * L::kStage, b = a + L::kA;
-#pragma unroll
-      for (int ks = 0; ks < kGtBK / 16; ++ks)
-        tc_mma(tmem, tc_desc(a + ks * 256, 128, 512), tc_desc(b + ks * 256, 128, 512), L::kIdesc,
+      const int steps = min(kGtBK, k_end - k_begin - c * kGtBK) / 16;
+      for (int ks = 0; ks < steps; ++ks)
+        tc_mma(tmem, tc_desc(a + ks * 256, 128, kGtGroup), tc_desc(b + ks * 256, 128, kGtGroup), L::kIdesc,
                (c > 0 || ks > 0) ? 1u : 0u);
       tc_commit(sb + L::kBar + 8 * buf);
     }
@@ -547,14 +566,29 @@ __global__ void __launch_bounds__(kGtThreads, 1)
   if (!__syncthreads_and(done && ok) && tid == 0) atomicOr(err, 1u);
   tc_fence_after();
   if (done && ok) {
-    const int row = m0 + warp * 32 + lane;
-    const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);
+    // a warp reaches the tensor-memory lanes of its number mod 4; the two warps of a lane group share the columns
+    const int row0 = m0 + (warp & 3) * 32;
+    const uint32_t t_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    float(*patch)[33] = reinterpret_cast<float(*)[33]>(smem) + warp * 32;  // (every MMA that read it is done)
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
+    for (int c0 = (warp >> 2) * 32; c0 < BN; c0 += 64) {
       float v[32];
       tc_ld32(t_row + c0, v);
+      if constexpr (Epi::kByRow) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) epi(row, c0 + 2 * j, v[2 * j], v[2 * j + 1]);
+        for (int j = 0; j < 16; ++j) epi(row0 + lane, c0 + 2 * j, v[2 * j], v[2 * j + 1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) patch[lane][j] = v[j];
+        __syncwarp();
+        const int col = 2 * (lane & 15);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int r = 2 * j + (lane >> 4);
+          epi(row0 + r, c0 + col, patch[r][col], patch[r][col + 1]);
+        }
+        __syncwarp();
+      }
     }
   }
   tc_fence_before();
