@@ -300,7 +300,7 @@ int clsph_gpu_counters(clsph_gpu* h, uint64_t* out3);
  * (the 4 x 8-bit LSD radix sort) on caller buffers: keys_out receives the
  * keys in ascending order, perm_out[s] the input index of sorted slot s
  * (equal keys keep input order). keys_in must not overlap the outputs.
- * Scratch comes from one 8.3 MB file-scope __device__ array held by every GPU
+ * Scratch comes from one 9.4 MB file-scope __device__ array held by every GPU
  * that loads the library until exit; n above 1,048,576 is rejected with
  * CLSPH_ERR_TOO_LARGE. All calls share that array (each clears what must
  * start at zero): calls whose GPU work overlaps race, so serialise them. The

@@ -40,7 +40,7 @@ int fail(int code, const std::string& msg) {
 }
 
 const char* kKernelNames[K_NUM_CLASSES] = {
-    "grid_setup", "keys",       "radix_hist",  "radix_sweep",    "gather",
+    "grid_setup", "keys",       "radix_sort",  "gather",
     "density",    "forces",     "advect",      "unpack_aos",     "pack_aos",      "misc",
     "features",   "mlp",        "learned_advect", "gate"};
 
@@ -115,18 +115,14 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
   h->launch(K_GRID_SETUP, k_grid_setup, dim3(1), dim3(256), h->bbox, h->grids,
             (const float*)h->scene_h, h->nscenes, h->status, h->digit_total, h->step_counters,
             h->ctl);
-  // k_keys also clears the cell index (slots is a power of two >= 1024)
-  h->launch(K_KEYS, k_keys, dim3(blocks), dim3(kBlock), (const float4*)h->st[0].pos, n,
-            (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, h->ctl, h->keys,
-            reinterpret_cast<uint4*>(h->ci.keys), h->slots / 4u);
+  // k_keys also clears the cell index (slots is a power of two >= 1024) and the sort's look-back words
+  h->launch(K_KEYS, k_keys, dim3(grid_blocks(n, h->sm_count * 6)), dim3(kBlock), (const float4*)h->st[0].pos, n,
+            (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, h->ctl, h->keys, h->digit_total,
+            reinterpret_cast<uint4*>(h->lookback), h->ntiles, reinterpret_cast<uint4*>(h->ci.keys), h->slots / 4u);
   if (until <= CLSPH_STAGE_GRID) return 0;
-  h->launch(K_RADIX_HIST, k_radix_hist, dim3(grid_blocks((n + 3) / 4, h->sm_count * 4)), dim3(kRadixThreads),
-            (const uint32_t*)h->keys, n, cctl, h->digit_total, h->lookback, h->ntiles);
-  for (int pass = 0; pass < 4; ++pass)
-    h->launch(K_RADIX_SWEEP, k_radix_onesweep, dim3(h->ntiles), dim3(kRadixThreads), h->keys, h->vals, n,
-              pass, cctl, (const uint32_t*)h->digit_total, h->lookback, h->ntiles,
-              h->step_counters + kCntRadixTile + pass, h->status, h->radix_spin_limit,
-              h->radix_withheld_tile);
+  h->launch(K_RADIX_SORT, k_radix_sort, dim3(std::min(h->ntiles, h->sm_count * 2)), dim3(kRadixThreads), h->keys,
+            h->vals, n, cctl, (const uint32_t*)h->digit_total, h->lookback, h->ntiles, h->step_counters + kCntRadix,
+            h->status, h->radix_spin_limit, h->radix_withheld_tile);
   const int src_ids = h->ids_sel, dst_ids = h->ids_sel ^ 1;
   h->launch(K_GATHER, k_gather, dim3(blocks), dim3(kBlock), n, (const DevGrid*)h->grids,
             (const uint16_t*)h->scene_of, h->ctl, (const uint32_t*)h->keys,

@@ -31,8 +31,7 @@ int fail(int code, const std::string& msg);
 enum KernelClass {
   K_GRID_SETUP,
   K_KEYS,
-  K_RADIX_HIST,
-  K_RADIX_SWEEP,
+  K_RADIX_SORT,
   K_GATHER,
   K_DENSITY,
   K_FORCES,

@@ -27,30 +27,22 @@
 
 #include "clsph_common.cuh"
 #include "clsph_mesh.cuh"
+#include "clsph_radix.cuh"
 
 namespace clsph {
 
 constexpr int kBlock = 256;
-// 2048-key tiles: 512 blocks per pass at 1M keys (4096-key tiles gave 256
-// blocks, 20 % warp occupancy and an 80-register scatter; 9-14 % slower)
-constexpr int kRadixThreads = 256;
-constexpr int kRadixItems = 8;
-constexpr int kRadixTile = kRadixThreads * kRadixItems;  // 2048 keys per tile
-constexpr int kRadixWarps = kRadixThreads / 32;
-constexpr int kRadixWarpSpan = kRadixTile / kRadixWarps;  // 256 keys per warp
-
 // per-substep counters, zeroed by k_grid_setup
 constexpr int kStepCounters = 8;
 // [kCntCells] occupied cells listed by k_gather, [kCntWorkDensity] cells
-// taken by the cell-warp density search, [kCntRadixTile + p] tiles taken by
-// radix pass p
-enum : int { kCntCells = 0, kCntWorkDensity = 1, kCntRadixTile = 4 };
+// taken by the cell-warp density search, [kCntRadix] the radix sort's ticket
+// and the tiles done of its passes (kRadixMaxPasses words)
+enum : int { kCntCells = 0, kCntWorkDensity = 1, kCntRadix = 4 };
 
 enum : uint32_t {
   kFlagGridOverflow = 1u,
   kFlagCollisionCap = 2u,
   kFlagNonFinite = 4u,
-  kFlagSortStall = 1u << 16,  // internal: a radix look-back wait ran out
 };
 
 struct DevGrid {         // one scene's grid of the current substep
@@ -62,17 +54,6 @@ struct DevGrid {         // one scene's grid of the current substep
   float half_margin;    // rounding margin of the half-cell tests, in cells
   uint32_t pad_[4];
 };
-
-// 8-bit radix passes that cover every key of the substep.
-__host__ __device__ __forceinline__ uint32_t radix_passes(uint32_t maxkey) {
-  uint32_t k = maxkey | 1u, bits = 0;
-  while (k) { ++bits; k >>= 1; }
-  return (bits + 7u) / 8u;
-}
-// Ping-pong buffer that holds the sorted keys and slots after all passes.
-__host__ __device__ __forceinline__ uint32_t sorted_sel(uint32_t maxkey) {
-  return radix_passes(maxkey) & 1u;
-}
 
 // Sort control block of a substep (device memory): [0] largest key,
 // [1] Morton bits (widest grid of all scenes), [2] scene bits, [3] nonzero when
@@ -406,265 +387,78 @@ static __global__ void k_pack_aos(float4* __restrict__ aos, uint32_t n, State st
   }
 }
 
-// Morton key per particle (grid.cl:56-66) and the largest key.
-__device__ __forceinline__ void keys_block(uint32_t vb, const float4* __restrict__ pos, uint32_t n,
-                                           const DevGrid* __restrict__ grids,
-                                           const uint16_t* __restrict__ scene_of, uint32_t* __restrict__ ctl,
-                                           uint32_t* __restrict__ keys, uint32_t& block_max) {
-  const KeySplit split{ctl[kCtlShift]};
-  if (threadIdx.x == 0) block_max = 0u;
-  __syncthreads();
-  const uint32_t i = vb * blockDim.x + threadIdx.x;
-  uint32_t key = 0u;
-  if (i < n) {
-    const uint32_t sc = scene_of[i];
-    const DevGrid& g = grids[sc];
-    const float4 p = pos[i];
-    uint32_t cx = __float2uint_rz(XDIV(XSUB(p.x, g.lo[0]), g.cell));
-    uint32_t cy = __float2uint_rz(XDIV(XSUB(p.y, g.lo[1]), g.cell));
-    uint32_t cz = __float2uint_rz(XDIV(XSUB(p.z, g.lo[2]), g.cell));
-    key = morton3(cx, cy, cz) | split.scene_bits(sc);
-    keys[i] = key;
-  }
-  key = __reduce_max_sync(0xFFFFFFFFu, key);
-  if ((threadIdx.x & 31) == 0) atomicMax(&block_max, key);
-  __syncthreads();
-  if (threadIdx.x == 0) atomicMax(&ctl[kCtlMaxKey], block_max);
-}
-
-// Also clears the cell index for this substep's k_gather (16 bytes a thread,
-// grid-stride), which no kernel between the two reads.
-static __global__ void __launch_bounds__(kBlock)
-    k_keys(const float4* __restrict__ pos, uint32_t n, const DevGrid* __restrict__ grids,
-           const uint16_t* __restrict__ scene_of, uint32_t* __restrict__ ctl,
-           uint32_t* __restrict__ keys, uint4* __restrict__ index_keys, uint32_t index_quads) {
-  __shared__ uint32_t block_max;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < index_quads; q += gridDim.x * blockDim.x)
-    index_keys[q] = make_uint4(0u, 0u, 0u, 0u);
-  keys_block(blockIdx.x, pos, n, grids, scene_of, ctl, keys, block_max);
-}
-
-// ---------------------------------------------------------------- radix sort
-// Stable LSD radix sort of (key, slot) with 8-bit digits in one-sweep form:
-// k_radix_hist reads the keys once and counts the digits of every pass;
-// k_radix_onesweep (one launch per pass) ranks a 2048-key tile in shared
-// memory, publishes the tile's per-digit counts, finds the counts of all
-// earlier tiles by decoupled look-back (each digit's thread walks back over
-// the published words until it meets an inclusive prefix) and scatters.
-// Passes beyond radix_passes return at once, so the launch sequence is fixed
-// (graph-capturable) while the work follows the key width. Ping-pong: pass p
-// reads buffer p&1 and writes (p+1)&1.
-//
-// Look-back words (one per tile and digit, per pass): bits 30-31 the state
-// (0 not yet published, 1 the tile's own count, 2 the inclusive prefix of
-// all tiles up to it), bits 0-29 the value (n < 2^28). Tiles are numbered in
-// the order blocks start (an atomic ticket), so every tile a block waits for
-// belongs to a block that is already running and publishes without waiting
-// itself; the wait is bounded all the same (spin_limit, by default
-// kRadixLookbackSpins), and a wait that runs out raises kFlagSortStall, which
-// clsph_gpu_sync reports as an error. After a stall the offsets of the tiles
-// behind it are wrong, but every store stays in bounds (destinations >= n are
-// skipped, and the slots a pass leaves unwritten keep earlier in-range
-// values), so the context stays usable.
-//
-// withheld_tile (a test hook of clsph_gpu_set_wait_limits; kNoTile in normal
-// use): that tile never publishes its words, so the tile after it waits on a
-// word that nothing sets until its spin limit runs out.
-constexpr uint32_t kRadixLookbackSpins = 1u << 20;
-constexpr uint32_t kNoTile = 0xFFFFFFFFu;
-constexpr uint32_t kLbAggregate = 1u << 30, kLbInclusive = 2u << 30, kLbValue = (1u << 30) - 1u;
-
-__device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed_gpu(uint32_t* p, uint32_t v) {
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
-
-// Digit counts of every pass in one read of the keys (16-byte loads), and the
-// look-back words of this substep's passes cleared.
-__device__ __forceinline__ void radix_hist_blocks(uint32_t blk, uint32_t nblk, const uint32_t* __restrict__ keys,
-                                                  uint32_t n, const uint32_t* __restrict__ ctl,
-                                                  uint32_t* __restrict__ digit_total,
-                                                  uint32_t* __restrict__ lookback, uint32_t ntiles,
-                                                  uint32_t (&hist)[4][256]) {
-  const uint32_t passes = radix_passes(ctl[kCtlMaxKey]);
-  for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) hist[i >> 8][i & 255] = 0u;
-  const size_t gtid = (size_t)blk * blockDim.x + threadIdx.x;
-  const size_t gstride = (size_t)nblk * blockDim.x;
-  const size_t words = (size_t)passes * ntiles * 256u;
-  for (size_t i = gtid; i < words; i += gstride) lookback[i] = 0u;
-  __syncthreads();
-  auto count = [&](uint32_t key) {
-    for (uint32_t p = 0; p < passes; ++p) atomicAdd(&hist[p][(key >> (8 * p)) & 0xFFu], 1u);
-  };
-  const uint32_t n4 = n / 4u;
-  for (size_t q = gtid; q < n4; q += gstride) {
-    const uint4 k = __ldg(reinterpret_cast<const uint4*>(keys) + q);
-    count(k.x);
-    count(k.y);
-    count(k.z);
-    count(k.w);
-  }
-  if (gtid < (n & 3u)) count(__ldg(&keys[4u * n4 + gtid]));
-  __syncthreads();
-  for (uint32_t p = 0; p < passes; ++p) {
-    const uint32_t c = hist[p][threadIdx.x];
-    if (c) atomicAdd(&digit_total[p * 256 + threadIdx.x], c);
-  }
-}
-
-static __global__ void __launch_bounds__(kRadixThreads)
-    k_radix_hist(const uint32_t* __restrict__ keys, uint32_t n, const uint32_t* __restrict__ ctl,
-                 uint32_t* __restrict__ digit_total, uint32_t* __restrict__ lookback, uint32_t ntiles) {
-  __shared__ uint32_t hist[4][256];
-  radix_hist_blocks(blockIdx.x, gridDim.x, keys, n, ctl, digit_total, lookback, ntiles, hist);
-}
-
-struct RadixSmem {
-  uint32_t cnt[kRadixWarps][256];
-  uint32_t hist[256];
-  uint32_t tile_off[256];
-  uint32_t warp_sums[kRadixWarps];
-  uint32_t tile_s;
+// Morton key per particle (grid.cl:56-66), the largest key and the digit
+// counts of the sort's passes. Also clears the sort's look-back words and the
+// cell index for this substep's k_gather (16 bytes a thread), which no kernel
+// between reads.
+struct KeysSmem {
+  uint32_t hist[kRadixMaxPasses][256];
+  uint32_t block_max;
 };
 
-// One tile of one radix pass: takes the next tile number from the ticket;
-// returns false (the whole block) once every tile of the pass is taken.
-__device__ __forceinline__ bool radix_sweep_tile(uint32_t* __restrict__ keys_base, uint32_t* __restrict__ vals_base,
-                                                 uint32_t n, int pass, const uint32_t* __restrict__ digit_total,
-                                                 uint32_t* __restrict__ lookback, uint32_t ntiles,
-                                                 uint32_t* __restrict__ tile_ticket, uint32_t* __restrict__ status,
-                                                 uint32_t spin_limit, uint32_t withheld_tile, RadixSmem& sm) {
-  auto& cnt = sm.cnt;
-  auto& hist = sm.hist;
-  auto& tile_off = sm.tile_off;
-  auto& warp_sums = sm.warp_sums;
-  uint32_t& tile_s = sm.tile_s;
-  __syncthreads();  // the block's previous tile is done with the shared arrays
-  const uint32_t* keys_in = keys_base + (size_t)(pass & 1) * n;
-  uint32_t* keys_out = keys_base + (size_t)((pass + 1) & 1) * n;
-  const uint32_t* vals_in = vals_base + (size_t)(pass & 1) * n;
-  uint32_t* vals_out = vals_base + (size_t)((pass + 1) & 1) * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) tile_s = atomicAdd(tile_ticket, 1u);
-  for (int w = 0; w < kRadixWarps; ++w) cnt[w][threadIdx.x] = 0u;
-  hist[threadIdx.x] = 0u;
+__device__ __forceinline__ void keys_blocks(uint32_t blk, uint32_t nblk, const float4* __restrict__ pos, uint32_t n,
+                                            const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
+                                            uint32_t* __restrict__ ctl, uint32_t* __restrict__ keys,
+                                            uint32_t* __restrict__ digit_total, uint4* __restrict__ lookback,
+                                            uint32_t ntiles, uint4* __restrict__ index_keys, uint32_t index_quads,
+                                            KeysSmem& sm) {
+  const KeySplit split{ctl[kCtlShift]};
+  // no key has more bits than the widest grid's keys and the scenes
+  const uint32_t passes = (min(split.shift + ctl[kCtlSceneBits], 32u) + 7u) / 8u;
+  const uint32_t first = blk * blockDim.x + threadIdx.x, stride = nblk * blockDim.x;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t q = first; q < index_quads; q += stride) index_keys[q] = zero;
+  for (uint32_t q = first; q < passes * ntiles * 64u; q += stride) lookback[q] = zero;
+  for (uint32_t q = threadIdx.x; q < kRadixMaxPasses * 256u; q += blockDim.x) sm.hist[q >> 8][q & 255u] = 0u;
+  if (threadIdx.x == 0) sm.block_max = 0u;
   __syncthreads();
-  const uint32_t tile = tile_s;
-  if (tile >= ntiles) return false;
-  const int shift = 8 * pass;
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t base = tile * kRadixTile + warp * kRadixWarpSpan;
-  uint32_t key[kRadixItems], val[kRadixItems], rank[kRadixItems];
-  // the tile's keys and its digit counts, published before the ranking so
-  // that later tiles' look-back finds them as early as possible
-#pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
-    const uint32_t idx = base + r * 32 + lane;
-    const bool valid = idx < n;
-    key[r] = valid ? keys_in[idx] : 0u;
-    val[r] = valid ? (pass == 0 ? idx : vals_in[idx]) : 0u;
-    if (valid) atomicAdd(&hist[(key[r] >> shift) & 0xFFu], 1u);
-  }
-  __syncthreads();
-  const uint32_t d = threadIdx.x;  // this thread's digit in the look-back and the offsets
-  const uint32_t local = hist[d];  // the tile's count of digit d
-  uint32_t* lb = lookback + (size_t)pass * ntiles * 256u;
-  const bool publish = tile != withheld_tile;
-  if (publish) st_relaxed_gpu(&lb[(size_t)tile * 256u + d], (tile == 0 ? kLbInclusive : kLbAggregate) | local);
-  // ranks within the tile: per warp in key order (rows of 32), then warps in order
-#pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
-    const uint32_t idx = base + r * 32 + lane;
-    const bool valid = idx < n;
-    const uint32_t dr = valid ? ((key[r] >> shift) & 0xFFu) : 256u;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, dr);
-    uint32_t rk = 0;
-    if (valid) rk = cnt[warp][dr] + __popc(peers & lt_mask);
-    __syncwarp();
-    if (valid && (peers & lt_mask) == 0u) cnt[warp][dr] += __popc(peers);
-    __syncwarp();
-    rank[r] = valid ? ((rk << 8) | dr) : 0xFFFFFFFFu;
-  }
-  uint32_t excl = 0;  // digit d in all earlier tiles
-  if (tile > 0) {
-    // walk back kLookbackWindow tiles per round (independent loads), adding
-    // published counts until an inclusive prefix (tile 0 always has one)
-    constexpr int kLookbackWindow = 4;
-    int64_t t = (int64_t)tile - 1;
-    uint32_t spins = 0;
-    bool done = false;
-    while (!done) {
-      uint32_t w[kLookbackWindow];
-#pragma unroll
-      for (int k = 0; k < kLookbackWindow; ++k)
-        w[k] = t - k >= 0 ? ld_relaxed_gpu(&lb[(size_t)(t - k) * 256u + d]) : kLbInclusive;
-      int used = 0;
-#pragma unroll
-      for (int k = 0; k < kLookbackWindow; ++k) {
-        if (done || used < k) break;       // stopped at an earlier word of this round
-        if ((w[k] & ~kLbValue) == 0u) break;  // not published yet: load it again
-        excl += w[k] & kLbValue;
-        ++used;
-        if (w[k] & kLbInclusive) done = true;
-      }
-      t -= used;
-      if (!done && used == 0) {
-        if (++spins > spin_limit) {
-          atomicOr(status, kFlagSortStall);
-          break;
-        }
-        __nanosleep(32);
-      }
+  uint32_t top = 0u;
+  for (uint32_t i = first; (i & ~31u) < n; i += stride) {
+    uint32_t key = 0u;
+    if (i < n) {
+      const uint32_t sc = scene_of[i];
+      const DevGrid& g = grids[sc];
+      const float4 p = pos[i];
+      const uint32_t cx = __float2uint_rz(XDIV(XSUB(p.x, g.lo[0]), g.cell));
+      const uint32_t cy = __float2uint_rz(XDIV(XSUB(p.y, g.lo[1]), g.cell));
+      const uint32_t cz = __float2uint_rz(XDIV(XSUB(p.z, g.lo[2]), g.cell));
+      key = morton3(cx, cy, cz) | split.scene_bits(sc);
+      keys[i] = key;
+      top = max(top, key);
     }
-    if (publish) st_relaxed_gpu(&lb[(size_t)tile * 256u + d], kLbInclusive | (excl + local));
+    radix_count(key, i < n, passes, sm.hist);
   }
+  top = __reduce_max_sync(0xFFFFFFFFu, top);
+  if ((threadIdx.x & 31) == 0) atomicMax(&sm.block_max, top);
   __syncthreads();
-  {  // per digit: exclusive prefix over warps
-    uint32_t run = 0;
-    for (int w = 0; w < kRadixWarps; ++w) {
-      const uint32_t c = cnt[w][d];
-      cnt[w][d] = run;
-      run += c;
-    }
-  }
-  // keys with a smaller digit: exclusive scan of the pass's digit totals
-  const uint32_t tot = digit_total[pass * 256 + d];
-  uint32_t x = tot;
-  for (int off = 1; off < 32; off <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
-    if (lane >= off) x += y;
-  }
-  if (lane == 31) warp_sums[warp] = x;
-  __syncthreads();
-  uint32_t below = x - tot;
-  for (int w = 0; w < warp; ++w) below += warp_sums[w];
-  tile_off[d] = below + excl;
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
-    if (rank[r] == 0xFFFFFFFFu) continue;
-    const uint32_t dd = rank[r] & 0xFFu;
-    const uint32_t dst = tile_off[dd] + cnt[warp][dd] + (rank[r] >> 8);
-    if (dst >= n) continue;  // only after a look-back wait ran out (flagged)
-    keys_out[dst] = key[r];
-    vals_out[dst] = val[r];
-  }
-  return true;
+  if (threadIdx.x == 0) atomicMax(&ctl[kCtlMaxKey], sm.block_max);
+  radix_count_flush(sm.hist, passes, digit_total);
+}
+
+static __global__ void __launch_bounds__(kBlock)
+    k_keys(const float4* __restrict__ pos, uint32_t n, const DevGrid* __restrict__ grids,
+           const uint16_t* __restrict__ scene_of, uint32_t* __restrict__ ctl, uint32_t* __restrict__ keys,
+           uint32_t* __restrict__ digit_total, uint4* __restrict__ lookback, uint32_t ntiles,
+           uint4* __restrict__ index_keys, uint32_t index_quads) {
+  __shared__ KeysSmem sm;
+  keys_blocks(blockIdx.x, gridDim.x, pos, n, grids, scene_of, ctl, keys, digit_total, lookback, ntiles, index_keys,
+              index_quads, sm);
+}
+
+// The sort of the substep's keys (clsph_radix.cuh): pass p reads buffer p & 1
+// and writes the other.
+__device__ __forceinline__ RadixBuffers substep_buffers(uint32_t* keys, uint32_t* vals, uint32_t n) {
+  return RadixBuffers{keys, keys, keys + n, vals, vals + n, 0u};
 }
 
 static __global__ void __launch_bounds__(kRadixThreads)
-    k_radix_onesweep(uint32_t* __restrict__ keys_base, uint32_t* __restrict__ vals_base, uint32_t n,
-                     int pass, const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ digit_total,
-                     uint32_t* __restrict__ lookback, uint32_t ntiles, uint32_t* __restrict__ tile_ticket,
-                     uint32_t* __restrict__ status, uint32_t spin_limit, uint32_t withheld_tile) {
-  if ((uint32_t)pass >= radix_passes(ctl[kCtlMaxKey])) return;
-  __shared__ RadixSmem sm;
-  radix_sweep_tile(keys_base, vals_base, n, pass, digit_total, lookback, ntiles, tile_ticket, status,
-                   spin_limit, withheld_tile, sm);
+    k_radix_sort(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
+                 const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ digit_total,
+                 uint32_t* __restrict__ lookback, uint32_t ntiles, uint32_t* __restrict__ counters,
+                 uint32_t* __restrict__ status, uint32_t spin_limit, uint32_t withheld_tile) {
+  __shared__ RadixSmem<kRadixThreads> sm;
+  radix_sort_blocks<kRadixThreads>(substep_buffers(keys, vals, n), n, radix_passes(ctl[kCtlMaxKey]), digit_total,
+                                   lookback, ntiles, counters, status, spin_limit, withheld_tile, sm);
 }
 
 // Half codes as bit planes: word [g * kHalfPlanes + b] holds bit b of the half

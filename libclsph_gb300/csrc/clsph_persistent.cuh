@@ -4,7 +4,7 @@
 // One block of 256 threads per resident slot on every SM (all co-resident,
 // which the cooperative launch guarantees) runs every phase of a substep in
 // turn, S substeps per launch, with a grid-wide barrier between phases:
-//   grid set-up (block 0) + cell-index clear | keys | digit counts |
+//   grid set-up (block 0) | keys, digit counts, cell-index clear |
 //   radix passes (tiles by ticket, decoupled look-back) | gather |
 //   density (two warps per occupied cell, 4 teams a block) | forces | advection
 // Each phase is the block-level body of the corresponding kernel of
@@ -59,8 +59,8 @@ struct PersistArgs {
 using PersistTeam = CellTeamSmem<2, 128, 14>;
 
 union PersistSmem {
-  RadixSmem radix;
-  uint32_t hist[4][256];
+  RadixSmem<kPersistThreads> radix;
+  KeysSmem keys;
   PersistTeam dens[kPersistThreads / 64];  // one team of two warps for each 64 threads
   GatherSmem gather;
   BboxSmem bbox;
@@ -68,12 +68,6 @@ union PersistSmem {
 };
 // dynamic shared memory: three resident blocks of the SM's 227 KB
 static_assert(sizeof(PersistSmem) <= 74 * 1024, "shared memory of the persistent kernel");
-
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 
 // Grid-wide barrier; false (for the whole block) when this block's wait ran
 // out or when it is the test hook's withheld block (which leaves at once,
@@ -122,26 +116,19 @@ static __global__ void __launch_bounds__(kPersistThreads, 3)
   const uint32_t nblk = (n + kPersistThreads - 1) / kPersistThreads;
   for (uint32_t s = 0; s < substeps; ++s) {
     const uint32_t src_ids = (ids_sel0 + s) & 1u;
-    // grid set-up of every scene, and an empty cell index
+    // grid set-up of every scene
     if (blockIdx.x == 0)
       grid_setup_block(a.bbox, a.grids, a.scene_h, a.nscenes, a.status, a.digit_total, a.step_counters, a.ctl,
                        sm.word);
-    for (uint32_t k = gtid; k < a.slots; k += gstride) a.ci.keys[k] = 0u;
     if (!grid_barrier(a, ok_s)) return;
-    for (uint32_t vb = blockIdx.x; vb < nblk; vb += gridDim.x)
-      keys_block(vb, a.st[0].pos, n, a.grids, a.scene_of, a.ctl, a.keys, sm.word);
+    keys_blocks(blockIdx.x, gridDim.x, a.st[0].pos, n, a.grids, a.scene_of, a.ctl, a.keys, a.digit_total,
+                reinterpret_cast<uint4*>(a.lookback), a.ntiles, reinterpret_cast<uint4*>(a.ci.keys), a.slots / 4u,
+                sm.keys);
     if (!grid_barrier(a, ok_s)) return;
-    radix_hist_blocks(blockIdx.x, gridDim.x, a.keys, n, a.ctl, a.digit_total, a.lookback, a.ntiles, sm.hist);
+    radix_sort_blocks<kPersistThreads>(substep_buffers(a.keys, a.vals, n), n, radix_passes(a.ctl[kCtlMaxKey]),
+                                       a.digit_total, a.lookback, a.ntiles, a.step_counters + kCntRadix, a.status,
+                                       a.spin_limit, a.withheld_tile, sm.radix);
     if (!grid_barrier(a, ok_s)) return;
-    const uint32_t passes = radix_passes(a.ctl[kCtlMaxKey]);
-    for (int pass = 0; pass < 4; ++pass) {
-      if ((uint32_t)pass >= passes) break;  // the same for every block
-      while (radix_sweep_tile(a.keys, a.vals, n, pass, a.digit_total, a.lookback, a.ntiles,
-                              a.step_counters + kCntRadixTile + pass, a.status, a.spin_limit, a.withheld_tile,
-                              sm.radix)) {
-      }
-      if (!grid_barrier(a, ok_s)) return;
-    }
     for (uint32_t vb = blockIdx.x; vb < nblk; vb += gridDim.x)
       gather_block(vb, n, a.grids, a.scene_of, a.ctl, a.keys, a.vals, a.st[0], a.st[1], a.ids[src_ids],
                    a.ids[src_ids ^ 1u], a.ci, a.cell_list, a.step_counters + kCntCells, a.planes, sm.gather);
