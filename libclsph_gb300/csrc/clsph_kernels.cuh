@@ -1040,7 +1040,8 @@ __device__ __forceinline__ uint32_t facing_slots(const uint32_t* __restrict__ pl
 #pragma unroll
   for (uint32_t b = 0; b < kHalfPlanes; b += 2) {  // an axis needs at most one of its two bits
     const uint32_t both = (need >> b) & 3u;
-    if (both) m &= __ldg(&p[b + (both >> 1)]);
+    const uint32_t v = __ldg(&p[b + (both >> 1)]);  // (loaded in any case: the loads don't wait for one another)
+    m &= both ? v : 0xFFFFFFFFu;
   }
   const uint32_t w0 = 32u * w;
   if (s > w0) m &= 0xFFFFFFFFu << (s - w0);
@@ -1116,7 +1117,10 @@ __device__ __forceinline__ void density_cells_team(
         const uint32_t w0 = s >> 5, words = e > s && lane != 13u ? ((e - 1u) >> 5) - w0 + 1u : 0u;
         uint32_t m[3];
 #pragma unroll
-        for (uint32_t w = 0; w < 3u; ++w) m[w] = w < words ? facing_slots(planes, w0 + w, s, e, need) : 0u;
+        for (uint32_t w = 0; w < 3u; ++w) {
+          const bool on = w < words;
+          m[w] = facing_slots(planes, on ? w0 + w : 0u, on ? s : 0u, on ? e : 1u, need) & (on ? 0xFFFFFFFFu : 0u);
+        }
         if (count <= 32u) {  // only the neighbour cells in its particles' windows
           uint32_t any = 0;
           if (lane < kHalfPlanes)
@@ -1286,17 +1290,19 @@ __device__ __forceinline__ void density_cells_team(
       uint32_t tag = 0;
       float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
       if (found) pj = next(tag);
+      const float ch = c.h, cm = c.mass, c6 = c.poly6;
       for (uint32_t k = 0; k < found;) {
         uint32_t tagn = 0;
         float4 pn = pj;
         if (++k < found) pn = next(tagn);
         const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
         const float rr = near_norm(d);
-        if (rr < c.h) {
-          rho = XADD(rho, poly6_term(rr, hh, c));
-          if (kept < nlist_cap) __stcs(list + (uint64_t)kept * n, (uint16_t)tag);
-          ++kept;
-        }
+        const bool hit = rr < ch;
+        const float qq = XSUB(hh, XMUL(rr, rr));
+        const float sum = XADD(rho, XMUL(cm, XMUL(c6, XMUL(XMUL(qq, qq), qq))));
+        rho = hit ? sum : rho;
+        if (hit && kept < nlist_cap) __stcs(list + (uint64_t)kept * n, (uint16_t)tag);
+        kept += hit ? 1u : 0u;
         tag = tagn;
         pj = pn;
       }
