@@ -108,6 +108,11 @@ void choose_shapes(clsph_gpu* h) {
 
 }  // namespace
 
+// Particles up to which the forces take eight and four lanes each. Measured (us, eight / four / one lane):
+// water on a floor 4,096 10 / 13 / 19; 14,000 11 / 14 / 19; 20,000 14.3 / 14.4 / 20; 32,768 18 / 17 / 20;
+// 45,000 21 / 22 / 20; 65,536 27 / 25 / 21.
+constexpr uint32_t kWide8 = 18000, kWide4 = 40000;
+
 int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
   const uint32_t n = h->n;
   const uint32_t blocks = grid_blocks(n);
@@ -183,7 +188,15 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
                 (const uint32_t*)h->ncount, h->nlist_cap, h->acc, NoForceHook{}, (const float4*)h->frec,
                 (const uint32_t*)h->nb_start);
     };
-    if (b == 64) args(k_forces<64>);
+    auto wide = [&](auto kernel, uint32_t lanes) {
+      h->launch(K_FORCES, kernel, dim3((n * lanes + kWideThreads - 1) / kWideThreads), dim3(kWideThreads), n,
+                (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, cctl, (const uint32_t*)h->keys, h->st[1],
+                (const float4*)h->aux, h->ci, (const Consts*)h->consts, (const uint16_t*)h->nlist,
+                (const uint32_t*)h->ncount, h->nlist_cap, h->acc, (const float4*)h->frec, (const uint32_t*)h->nb_start);
+    };
+    if (n <= kWide8) wide(k_forces_wide<8>, 8);
+    else if (n <= kWide4) wide(k_forces_wide<4>, 4);
+    else if (b == 64) args(k_forces<64>);
     else if (b == 256) args(k_forces<256>);
     else args(k_forces<128>);
   }
