@@ -117,19 +117,28 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
   const uint32_t n = h->n;
   const uint32_t blocks = grid_blocks(n);
   const uint32_t* cctl = h->ctl;
-  h->launch(K_GRID_SETUP, k_grid_setup, dim3(1), dim3(256), h->bbox, h->grids,
+  // Every kernel but two may have its blocks placed under the tail of the one
+  // before it. The cell search takes an SM's whole shared memory: blocks of the
+  // forces placed beside it find the SM's L1 cache at its smallest and keep it
+  // so (1,048,576 particles: a frame 6.24 -> 7.85 ms), and blocks of the search
+  // beside the gather fit an SM only after it is laid out anew. Both wait there.
+  // A callback substep of 4,096 particles: none / all but these two / all placed
+  // early 0.0938 / 0.0813 / 0.0787 ms of host time; a frame of 1,048,576
+  // 6.240 / 6.226 / 7.859.
+  const bool early = h->search == CLSPH_SEARCH_PARTICLE_WARPS;
+  h->launch_next(true, K_GRID_SETUP, k_grid_setup, dim3(1), dim3(256), h->bbox, h->grids,
             (const float*)h->scene_h, h->nscenes, h->status, h->digit_total, h->step_counters,
             h->ctl);
   // k_keys also clears the cell index (slots is a power of two >= 1024) and the sort's look-back words
-  h->launch(K_KEYS, k_keys, dim3(grid_blocks(n, h->sm_count * 6)), dim3(kBlock), (const float4*)h->st[0].pos, n,
+  h->launch_next(true, K_KEYS, k_keys, dim3(grid_blocks(n, h->sm_count * 6)), dim3(kBlock), (const float4*)h->st[0].pos, n,
             (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, h->ctl, h->keys, h->digit_total,
             reinterpret_cast<uint4*>(h->lookback), h->ntiles, reinterpret_cast<uint4*>(h->ci.keys), h->slots / 4u);
   if (until <= CLSPH_STAGE_GRID) return 0;
-  h->launch(K_RADIX_SORT, k_radix_sort, dim3(std::min(h->ntiles, h->sm_count * 2)), dim3(kRadixThreads), h->keys,
+  h->launch_next(true, K_RADIX_SORT, k_radix_sort, dim3(std::min(h->ntiles, h->sm_count * 2)), dim3(kRadixThreads), h->keys,
             h->vals, n, cctl, (const uint32_t*)h->digit_total, h->lookback, h->ntiles, h->step_counters + kCntRadix,
             h->status, h->radix_spin_limit, h->radix_withheld_tile);
   const int src_ids = h->ids_sel, dst_ids = h->ids_sel ^ 1;
-  h->launch(K_GATHER, k_gather, dim3(blocks), dim3(kBlock), n, (const DevGrid*)h->grids,
+  h->launch_next(true, K_GATHER, k_gather, dim3(blocks), dim3(kBlock), n, (const DevGrid*)h->grids,
             (const uint16_t*)h->scene_of, h->ctl, (const uint32_t*)h->keys,
             (const uint32_t*)h->vals, h->st[0], h->st[1], (const uint32_t*)h->ids[src_ids],
             h->ids[dst_ids], h->ci, h->cell_list, h->step_counters + kCntCells, h->planes);
@@ -140,7 +149,7 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
     const int b = h->density_block == 64 ? 64 : 128;
     const dim3 grid((n + b - 1) / b);
     auto args = [&](auto kernel) {
-      h->launch(K_DENSITY, kernel, grid, dim3(b), n, (const DevGrid*)h->grids,
+      h->launch_next(early, K_DENSITY, kernel, grid, dim3(b), n, (const DevGrid*)h->grids,
                 (const uint16_t*)h->scene_of, cctl, (const uint32_t*)h->keys,
                 (const float4*)h->st[1].pos, h->ci, (const Consts*)h->consts, h->aux, h->nlist,
                 h->ncount, h->nlist_cap, (const float4*)h->st[1].vel, h->frec, h->nb_start);
@@ -154,7 +163,7 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
           per_sm = 1;
         resident = (uint32_t)per_sm * h->sm_count;
       }
-      h->launch(K_DENSITY, kernel, dim3(std::min(resident, n)), dim3(warps * 32),
+      h->launch_next(early, K_DENSITY, kernel, dim3(std::min(resident, n)), dim3(warps * 32),
                 n, (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, cctl,
                 (const uint32_t*)h->keys, (const float4*)h->st[1].pos, (const uint32_t*)h->planes, h->ci,
                 (const Consts*)h->consts, h->aux, h->nlist, h->ncount, h->nlist_cap,
@@ -167,7 +176,7 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
       else if (h->packed_cells) cells(k_density_cells<CellTeamSmem<2, 128, 14>, 12>, 1, 2);
       else cells(k_density_cells<CellTeamSmem<2, 92, 11>, 16>, 0, 2);
     } else if (h->search == CLSPH_SEARCH_PARTICLE_WARPS) {
-      h->launch(K_DENSITY, k_density_pwarp, dim3((n + kParticleWarps - 1) / kParticleWarps),
+      h->launch_next(early, K_DENSITY, k_density_pwarp, dim3((n + kParticleWarps - 1) / kParticleWarps),
                 dim3(kParticleWarps * 32), n, (const DevGrid*)h->grids, (const uint16_t*)h->scene_of,
                 cctl, (const uint32_t*)h->keys, (const float4*)h->st[1].pos, h->ci,
                 (const Consts*)h->consts, h->aux, h->nlist, h->ncount, h->nlist_cap,
@@ -182,14 +191,14 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
     const int b = h->forces_block;
     const dim3 grid((n + b - 1) / b);
     auto args = [&](auto kernel) {
-      h->launch(K_FORCES, kernel, grid, dim3(b), n, (const DevGrid*)h->grids,
+      h->launch_next(early, K_FORCES, kernel, grid, dim3(b), n, (const DevGrid*)h->grids,
                 (const uint16_t*)h->scene_of, cctl, (const uint32_t*)h->keys, h->st[1],
                 (const float4*)h->aux, h->ci, (const Consts*)h->consts, (const uint16_t*)h->nlist,
                 (const uint32_t*)h->ncount, h->nlist_cap, h->acc, NoForceHook{}, (const float4*)h->frec,
                 (const uint32_t*)h->nb_start);
     };
     auto wide = [&](auto kernel, uint32_t lanes) {
-      h->launch(K_FORCES, kernel, dim3((n * lanes + kWideThreads - 1) / kWideThreads), dim3(kWideThreads), n,
+      h->launch_next(early, K_FORCES, kernel, dim3((n * lanes + kWideThreads - 1) / kWideThreads), dim3(kWideThreads), n,
                 (const DevGrid*)h->grids, (const uint16_t*)h->scene_of, cctl, (const uint32_t*)h->keys, h->st[1],
                 (const float4*)h->aux, h->ci, (const Consts*)h->consts, (const uint16_t*)h->nlist,
                 (const uint32_t*)h->ncount, h->nlist_cap, h->acc, (const float4*)h->frec, (const uint32_t*)h->nb_start);
@@ -273,7 +282,7 @@ int clsph_host::launch_persistent(clsph_gpu* h, uint32_t substeps) {
 
 int clsph_host::enqueue_advect(clsph_gpu* h) {
   const uint32_t n = h->n;
-  h->launch(K_ADVECT, k_advect<false>, dim3(grid_blocks(n, h->sm_count * h->advect_blocks_per_sm)),
+  h->launch_next(true, K_ADVECT, k_advect<false>, dim3(grid_blocks(n, h->sm_count * h->advect_blocks_per_sm)),
             dim3(kBlock), n, h->st[1],
             (const float4*)h->acc, h->st[0], (const DevMesh*)h->meshes, (const Consts*)h->consts,
             (const uint16_t*)h->scene_of, h->max_iters, h->bbox, h->status, h->capped,

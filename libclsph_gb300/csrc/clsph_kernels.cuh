@@ -39,6 +39,19 @@ constexpr int kStepCounters = 8;
 // and the tiles done of its passes (kRadixMaxPasses words)
 enum : int { kCntCells = 0, kCntWorkDensity = 1, kCntRadix = 4 };
 
+// Opens every kernel of a substep: waits until the kernel launched before this
+// one has ended and its writes are visible, then lets the next one's blocks
+// start (they wait here in turn). A kernel launched by clsph_gpu::launch_next
+// so has its blocks on the SMs when its inputs are ready. A chain of such
+// kernels keeps its order, because each one ends only after its own wait;
+// launched in the plain way, both instructions do nothing. Always false: the
+// branch on it keeps the compiler from moving a load of read-only data up.
+__device__ __forceinline__ bool never_after_previous() {
+  uint32_t zero;
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
+  return zero != 0u;
+}
+
 enum : uint32_t {
   kFlagGridOverflow = 1u,
   kFlagCollisionCap = 2u,
@@ -240,6 +253,7 @@ static __global__ void k_grid_setup(uint32_t* __restrict__ bbox_all, DevGrid* __
                                     const float* __restrict__ scene_h, uint32_t nscenes,
                                     uint32_t* __restrict__ status, uint32_t* __restrict__ digit_total,
                                     uint32_t* __restrict__ step_counters, uint32_t* __restrict__ ctl) {
+  if (never_after_previous()) return;
   __shared__ uint32_t shift_s;
   grid_setup_block(bbox_all, grids, scene_h, nscenes, status, digit_total, step_counters, ctl, shift_s);
 }
@@ -440,6 +454,7 @@ static __global__ void __launch_bounds__(kBlock)
            const uint16_t* __restrict__ scene_of, uint32_t* __restrict__ ctl, uint32_t* __restrict__ keys,
            uint32_t* __restrict__ digit_total, uint4* __restrict__ lookback, uint32_t ntiles,
            uint4* __restrict__ index_keys, uint32_t index_quads) {
+  if (never_after_previous()) return;
   __shared__ KeysSmem sm;
   keys_blocks(blockIdx.x, gridDim.x, pos, n, grids, scene_of, ctl, keys, digit_total, lookback, ntiles, index_keys,
               index_quads, sm);
@@ -456,6 +471,7 @@ static __global__ void __launch_bounds__(kRadixThreads)
                  const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ digit_total,
                  uint32_t* __restrict__ lookback, uint32_t ntiles, uint32_t* __restrict__ counters,
                  uint32_t* __restrict__ status, uint32_t spin_limit, uint32_t withheld_tile) {
+  if (never_after_previous()) return;
   __shared__ RadixSmem<kRadixThreads> sm;
   radix_sort_blocks<kRadixThreads>(substep_buffers(keys, vals, n), n, radix_passes(ctl[kCtlMaxKey]), digit_total,
                                    lookback, ntiles, counters, status, spin_limit, withheld_tile, sm);
@@ -550,6 +566,7 @@ static __global__ void __launch_bounds__(kBlock)
              const uint32_t* __restrict__ ids_src, uint32_t* __restrict__ ids_dst,
              CellIndex ci, uint2* __restrict__ cell_list,
              uint32_t* __restrict__ cell_count, uint32_t* __restrict__ planes) {
+  if (never_after_previous()) return;
   __shared__ GatherSmem sm;
   gather_block(blockIdx.x, n, grids, scene_of, ctl, keys_base, vals_base, src, dst, ids_src, ids_dst, ci,
                cell_list, cell_count, planes, sm);
@@ -752,6 +769,7 @@ __global__ void __launch_bounds__(BLOCK)
               const Consts* __restrict__ consts, float4* __restrict__ aux_out,
               uint16_t* __restrict__ nlist, uint32_t* __restrict__ ncount, uint32_t nlist_cap,
               const float4* __restrict__ vel, float4* __restrict__ frec, uint32_t* __restrict__ nb_start) {
+  if (never_after_previous()) return;
   __shared__ uint16_t cand[kScanCap][BLOCK];  // tags of the cull's survivors
   __shared__ uint32_t cstart[27][BLOCK];      // first slot of each window cell
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -912,6 +930,7 @@ static __global__ void __launch_bounds__(kParticleWarps * 32)
                     float4* __restrict__ aux_out, uint16_t* __restrict__ nlist,
                     uint32_t* __restrict__ ncount, uint32_t nlist_cap, const float4* __restrict__ vel,
                     float4* __restrict__ frec, uint32_t* __restrict__ nb_start) {
+  if (never_after_previous()) return;
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;  // whole warps
   const KeySplit split{ctl[kCtlShift]};
@@ -1326,6 +1345,7 @@ __global__ void __launch_bounds__(Team::kWarps * 32, BLOCKS)
                     uint32_t nlist_cap, const float4* __restrict__ vel,
                     float4* __restrict__ frec, const uint2* __restrict__ cell_list,
                     uint32_t* __restrict__ counters, uint32_t* __restrict__ nb_start) {
+  if (never_after_previous()) return;
   __shared__ Team sm;
   density_cells_team(n, grids, ctl, scene_of, keys_base, pos, planes, ci, consts, aux_out, nlist, ncount, nlist_cap, vel,
                      frec, cell_list, counters, nb_start, sm, threadIdx.x >> 5, blockIdx.x, gridDim.x, 1u);
@@ -1508,6 +1528,7 @@ __global__ void __launch_bounds__(BLOCK, Hook::kPairs ? 640 / BLOCK : 1024 / BLO
              const uint32_t* __restrict__ ncount, uint32_t nlist_cap,
              float4* __restrict__ acc_out, Hook hook, const float4* __restrict__ frec,
              const uint32_t* __restrict__ nb_start) {
+  if (never_after_previous()) return;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if ((i & ~31u) >= n) return;  // whole warps
   forces_particle(i < n, i, n, grids, scene_of, ctl, keys_base, st, aux, ci, consts, nlist, ncount, nlist_cap,
@@ -1530,6 +1551,7 @@ static __global__ void __launch_bounds__(kWideThreads)
                   const uint16_t* __restrict__ nlist, const uint32_t* __restrict__ ncount, uint32_t nlist_cap,
                   float4* __restrict__ acc_out, const float4* __restrict__ frec,
                   const uint32_t* __restrict__ nb_start) {
+  if (never_after_previous()) return;
   __shared__ float terms[kWideThreads][kWideTerms + 1];
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u, l = lane & (LANES - 1u);
   if (((t & ~31u) / LANES) >= n) return;  // whole warps
@@ -1808,6 +1830,7 @@ __global__ void __launch_bounds__(kBlock, 4)
              uint32_t* __restrict__ status, unsigned long long* __restrict__ capped_count,
              const float4* __restrict__ corr, float dt_mult, float pos_w, const float4* __restrict__ aux,
              const float* __restrict__ y_stats) {
+  if (never_after_previous()) return;
   __shared__ BboxSmem bsm;
   advect_blocks<kLearned>(blockIdx.x, gridDim.x, n, in, acc, out, meshes, consts, scene_of, max_iters, bbox,
                           status, capped_count, corr, dt_mult, pos_w, aux, y_stats, bsm);

@@ -684,7 +684,7 @@ int enqueue_learned_tail(clsph_gpu* h, clsph_mlp* m, LearnedCache* L, uint32_t d
   rc = launch_tc(h->stream, h->sm_count, L->x, n, tc_weights(m), clsph_nn::StoreRaw{L->corr},
                  reinterpret_cast<uint32_t*>(L->dev_sum + kGateSums), h, K_MLP);
   if (rc) return rc;
-  h->launch(K_LEARNED_ADVECT, k_advect<true>, dim3(grid_blocks(n, h->sm_count * h->advect_blocks_per_sm)),
+  h->launch_next(true, K_LEARNED_ADVECT, k_advect<true>, dim3(grid_blocks(n, h->sm_count * h->advect_blocks_per_sm)),
             dim3(kBlock), n, h->st[1], (const float4*)h->acc, h->st[0], (const DevMesh*)h->meshes,
             (const Consts*)h->consts, (const uint16_t*)h->scene_of, h->max_iters, h->bbox, h->status,
             h->capped, (const float4*)L->corr, (float)dt_mult, position_weight(dt_mult),
