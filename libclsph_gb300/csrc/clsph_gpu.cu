@@ -722,9 +722,9 @@ int clsph_gpu_upload(clsph_gpu* h, const clsph_particle* particles) {
                              cudaMemcpyHostToDevice, h->stream));
     src = h->aos_stage;
   }
-  h->launch(K_MISC, k_bbox_reset, dim3(grid_blocks(6 * h->nscenes, 64)), dim3(kBlock), h->bbox,
+  h->launch_next(true, K_MISC, k_bbox_reset, dim3(grid_blocks(6 * h->nscenes, 64)), dim3(kBlock), h->bbox,
             h->nscenes);
-  h->launch(K_UNPACK, k_unpack_aos, aos_grid(h), dim3(kBlock), src, h->n, h->st[0],
+  h->launch_next(true, K_UNPACK, k_unpack_aos, aos_grid(h), dim3(kBlock), src, h->n, h->st[0],
             (const uint16_t*)h->scene_of, h->bbox, h->status);
   h->uploaded = true;
   h->partial = false;
@@ -736,7 +736,7 @@ int clsph_gpu_download(clsph_gpu* h, clsph_particle* particles) {
   if (!h || !particles) return fail(CLSPH_ERR_ARGUMENT, "download: bad argument");
   if (!h->uploaded || h->partial) return fail(CLSPH_ERR_STATE, "download: no complete state");
   float4* dst = static_cast<float4*>(mapped_host_records(particles));
-  h->launch(K_PACK, k_pack_aos, aos_grid(h), dim3(kBlock), dst ? dst : h->aos_stage, h->n, h->st[0],
+  h->launch_next(true, K_PACK, k_pack_aos, aos_grid(h), dim3(kBlock), dst ? dst : h->aos_stage, h->n, h->st[0],
             (const float4*)h->aux, (const uint32_t*)h->keys, (const uint32_t*)h->ctl,
             h->have_fields ? 1 : 0);
   if (!dst)

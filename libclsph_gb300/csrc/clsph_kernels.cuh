@@ -39,7 +39,7 @@ constexpr int kStepCounters = 8;
 // and the tiles done of its passes (kRadixMaxPasses words)
 enum : int { kCntCells = 0, kCntWorkDensity = 1, kCntRadix = 4 };
 
-// Opens every kernel of a substep: waits until the kernel launched before this
+// Opens the kernels of a substep and of the transfers: waits until the kernel launched before this
 // one has ended and its writes are visible, then lets the next one's blocks
 // start (they wait here in turn). A kernel launched by clsph_gpu::launch_next
 // so has its blocks on the SMs when its inputs are ready. A chain of such
@@ -259,6 +259,7 @@ static __global__ void k_grid_setup(uint32_t* __restrict__ bbox_all, DevGrid* __
 }
 
 static __global__ void k_bbox_reset(uint32_t* __restrict__ bbox, uint32_t nscenes) {
+  if (never_after_previous()) return;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < 6 * nscenes; k += gridDim.x * blockDim.x)
     bbox[k] = (k % 6) < 3 ? f2ord(2147483648.0f) : f2ord(-2147483648.0f);
 }
@@ -343,6 +344,7 @@ __device__ __forceinline__ void bbox_accumulate(float3 lo, float3 hi, int scene,
 static __global__ void k_unpack_aos(const float4* __restrict__ aos, uint32_t n, State st,
                              const uint16_t* __restrict__ scene_of, uint32_t* __restrict__ bbox,
                              uint32_t* __restrict__ status) {
+  if (never_after_previous()) return;
   const float qnan = __int_as_float(0x7FC00000);
   const size_t words = (size_t)n * 5;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -378,6 +380,7 @@ static __global__ void k_unpack_aos(const float4* __restrict__ aos, uint32_t n, 
 static __global__ void k_pack_aos(float4* __restrict__ aos, uint32_t n, State st,
                            const float4* __restrict__ aux, const uint32_t* __restrict__ keys_base,
                            const uint32_t* __restrict__ ctl, int have_fields) {
+  if (never_after_previous()) return;
   const KeySplit split{ctl[kCtlShift]};
   const uint32_t sel = have_fields ? sorted_sel(ctl[kCtlMaxKey]) : 0u;
   const uint32_t* keys = keys_base + (size_t)sel * n;
