@@ -210,20 +210,9 @@ struct clsph_gpu {
     launch_smem(cls, k, g, b, 0, args...);
   }
 
-  // A kernel that opens with never_after_previous(): if `early`, its blocks may
-  // be placed while the kernel before it still runs.
   template <typename Kernel, typename... Args>
   void launch_next(bool early, int cls, Kernel k, dim3 g, dim3 b, Args... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = early;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = g;
-    cfg.blockDim = b;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    timed(cls, [&] { cudaLaunchKernelEx(&cfg, k, args...); });
+    timed(cls, [&] { launch_early(k, g, b, 0, stream, early, args...); });
   }
 
   template <typename Kernel, typename... Args>

@@ -39,19 +39,6 @@ constexpr int kStepCounters = 8;
 // and the tiles done of its passes (kRadixMaxPasses words)
 enum : int { kCntCells = 0, kCntWorkDensity = 1, kCntRadix = 4 };
 
-// Opens the kernels of a substep and of the transfers: waits until the kernel launched before this
-// one has ended and its writes are visible, then lets the next one's blocks
-// start (they wait here in turn). A kernel launched by clsph_gpu::launch_next
-// so has its blocks on the SMs when its inputs are ready. A chain of such
-// kernels keeps its order, because each one ends only after its own wait;
-// launched in the plain way, both instructions do nothing. Always false: the
-// branch on it keeps the compiler from moving a load of read-only data up.
-__device__ __forceinline__ bool never_after_previous() {
-  uint32_t zero;
-  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
-  return zero != 0u;
-}
-
 enum : uint32_t {
   kFlagGridOverflow = 1u,
   kFlagCollisionCap = 2u,

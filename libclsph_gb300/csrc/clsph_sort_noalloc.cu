@@ -54,9 +54,16 @@ constexpr size_t kScratchWords = kOffCtl + 64;
 
 static __device__ __align__(256) uint32_t g_sort_scratch[kScratchWords];
 
+// Clears the digit totals and the control words, which lie side by side.
+__global__ void __launch_bounds__(kThreads) k_na_clear(uint32_t* __restrict__ scratch) {
+  if (never_after_previous()) return;
+  for (size_t q = kOffTotals + threadIdx.x; q < kScratchWords; q += kThreads) scratch[q] = 0u;
+}
+
 // Largest key and the digit counts of every pass; clears the look-back words.
 __global__ void __launch_bounds__(kThreads) k_na_count(const uint32_t* __restrict__ keys, uint32_t n, uint32_t ntiles,
                                                        uint32_t* __restrict__ scratch) {
+  if (never_after_previous()) return;
   __shared__ uint32_t hist[kRadixMaxPasses][256];
   __shared__ uint32_t block_max;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -82,6 +89,7 @@ __global__ void __launch_bounds__(kThreads) k_na_count(const uint32_t* __restric
 __global__ void __launch_bounds__(kRadixThreads)
     k_na_sort(const uint32_t* __restrict__ keys, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
               uint32_t n, uint32_t ntiles, uint32_t* __restrict__ scratch) {
+  if (never_after_previous()) return;
   __shared__ RadixSmem<kRadixThreads> sm;
   uint32_t* ctl = scratch + kOffCtl;
   const uint32_t passes = radix_passes(ctl[kMaxKey]);
@@ -143,12 +151,12 @@ extern "C" int clsph_gpu_sort_keys_noalloc(const uint32_t* keys_in, uint32_t* ke
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const uint32_t ntiles = (n + kRadixTile - 1) / kRadixTile;
-  // totals and control words lie side by side
-  if (cudaMemsetAsync(scratch + kOffTotals, 0, sizeof(uint32_t) * (kScratchWords - kOffTotals), s) == cudaSuccess) {
-    const uint32_t blocks = (n + kThreads - 1) / kThreads;
-    k_na_count<<<blocks < 608u ? blocks : 608u, kThreads, 0, s>>>(keys_in, n, ntiles, scratch);
-    k_na_sort<<<ntiles, kRadixThreads, 0, s>>>(keys_in, keys_out, perm_out, n, ntiles, scratch);
-  }
+  const uint32_t blocks = (n + kThreads - 1) / kThreads;
+  launch_early(k_na_clear, dim3(1), dim3(kThreads), 0, s, true, scratch);
+  launch_early(k_na_count, dim3(blocks < 608u ? blocks : 608u), dim3(kThreads), 0, s, true, keys_in, n, ntiles,
+               scratch);
+  launch_early(k_na_sort, dim3(ntiles), dim3(kRadixThreads), 0, s, true, keys_in, keys_out, perm_out, n, ntiles,
+               scratch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     clsph_set_last_error(std::string("sort_keys_noalloc: launch: ") + cudaGetErrorString(e));
