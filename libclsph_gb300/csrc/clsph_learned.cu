@@ -398,7 +398,8 @@ int gemm_tc(cudaStream_t s, uint32_t* err, const bf16* A, int lda, const bf16* B
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)clsph_nn::kGtSmem);
   if (e != cudaSuccess) return fail(CLSPH_ERR_CUDA, std::string("mlp: GEMM shared memory: ") + cudaGetErrorString(e));
   dim3 grid(1, M / clsph_nn::kGtRows, K / k_split);
-  kernel<<<grid, clsph_nn::kGtThreads, clsph_nn::kGtSmem, s>>>(A, lda, B, ldb, K, k_split, epi, err);
+  launch_early(kernel, grid, dim3(clsph_nn::kGtThreads), clsph_nn::kGtSmem, s, true, A, lda, B, ldb, K, k_split, epi,
+               err);
   return 0;
 }
 
@@ -469,13 +470,22 @@ int ensure_loss(clsph_mlp* m, uint32_t count) {
   return 0;
 }
 
+// The rows of a pass into m->xb / m->yb; with `backward`, m->grad is cleared.
+// The kernels of a pass are placed early (65,536 rows: a training pass 375 ->
+// 354 us; with the clear here rather than a memset between them 352).
+void gather_batch(clsph_mlp* m, const float* x_raw, const float* y_raw, const uint32_t* idx, uint32_t rows,
+                  bool backward) {
+  launch_early(clsph_nn::k_gather_batch, dim3((rows * (kIn + kOut) + 255) / 256), dim3(256), 0, m->stream, true, x_raw,
+               y_raw, idx, rows, (const float*)(m->blob + clsph_nn::kOffXMu), m->xb, m->yb,
+               backward ? m->grad : nullptr);
+}
+
 // Forward + loss (into *loss_slot) and, when `backward`, gradients into
-// m->grad for the `rows` rows already in m->xb / m->yb.
+// m->grad (cleared by gather_batch) for the `rows` rows already in m->xb / m->yb.
 int pass(clsph_mlp* m, uint32_t rows, float* loss_slot, bool backward) {
   cudaStream_t s = m->stream;
   const float* p = m->blob;
   int rc;
-  if (backward) CUDA_TRY(cudaMemsetAsync(m->grad, 0, sizeof(float) * kParams, s));
   uint32_t* err = m->err;
   // Z1 = X W1 + b1, H1 = GELU(Z1); the weights with K contiguous, so that both operands are copied as they lie
   if ((rc = gemm_tc<kHid, true, true>(s, err, m->xb, kIn, m->w1t, kIn, rows, kHid, kIn, kIn,
@@ -486,9 +496,10 @@ int pass(clsph_mlp* m, uint32_t rows, float* loss_slot, bool backward) {
                                       EpiHidden{p + clsph_nn::kOffB2, m->z2, m->h2, kHid, 2.f})))
     return rc;
   // Y = H2 W3 + b3, loss, dZ2, dW3, db3, db2
-  clsph_nn::k_head<<<std::min(rows / clsph_nn::kHeadWarps, 2 * m->sms), clsph_nn::kHeadWarps * 32, 0, s>>>(
-      m->h2, m->z2, p + clsph_nn::kOffW3, p + clsph_nn::kOffB3, m->yb, rows, 1.f / rows, m->dz2,
-      m->grad + clsph_nn::kOffW3, m->grad + clsph_nn::kOffB3, m->grad + clsph_nn::kOffB2, loss_slot);
+  launch_early(clsph_nn::k_head, dim3(std::min(rows / clsph_nn::kHeadWarps, 2 * m->sms)),
+               dim3(clsph_nn::kHeadWarps * 32), 0, s, true, m->h2, m->z2, p + clsph_nn::kOffW3,
+               p + clsph_nn::kOffB3, m->yb, rows, 1.f / rows, m->dz2, m->grad + clsph_nn::kOffW3,
+               m->grad + clsph_nn::kOffB3, m->grad + clsph_nn::kOffB2, loss_slot);
   if (!backward) return 0;
   const int splits = rows / kSplitK;
   const size_t split_stride = (size_t)kHid * kHid;
@@ -496,8 +507,8 @@ int pass(clsph_mlp* m, uint32_t rows, float* loss_slot, bool backward) {
   if ((rc = gemm_tc<kHid, false, false>(s, err, m->h1, kHid, m->dz2, kHid, kHid, kHid, rows, kSplitK,
                                         EpiPartial{m->ws, kHid, split_stride})))
     return rc;
-  clsph_nn::k_reduce_splits<<<(kHid * kHid + 255) / 256, 256, 0, s>>>(m->ws, splits, (size_t)kHid * kHid,
-                                                                      m->grad + clsph_nn::kOffW2);
+  launch_early(clsph_nn::k_reduce_splits, dim3((kHid * kHid + 255) / 256), dim3(256), 0, s, true, m->ws, splits,
+               (size_t)kHid * kHid, m->grad + clsph_nn::kOffW2);
   // dZ1 = (dZ2 W2^T) * GELU'(Z1)
   if ((rc = gemm_tc<kHid, true, true>(s, err, m->dz2, kHid, m->w2b, kHid, rows, kHid, kHid, kHid,
                                       EpiGeluGrad{m->z1, m->dz1, kHid})))
@@ -507,9 +518,10 @@ int pass(clsph_mlp* m, uint32_t rows, float* loss_slot, bool backward) {
   if ((rc = gemm_tc<kIn, false, false>(s, err, m->dz1, kHid, m->xb, kIn, kHid, kIn, rows, kSplitK,
                                        clsph_nn::EpiPartialT{m->ws, kHid, (size_t)kIn * kHid})))
     return rc;
-  clsph_nn::k_reduce_splits<<<(kIn * kHid + 255) / 256, 256, 0, s>>>(m->ws, splits, (size_t)kIn * kHid,
-                                                                    m->grad + clsph_nn::kOffW1);
-  clsph_nn::k_colsum<<<rows / 256, kHid, 0, s>>>(m->dz1, rows, 256, m->grad + clsph_nn::kOffB1);
+  launch_early(clsph_nn::k_reduce_splits, dim3((kIn * kHid + 255) / 256), dim3(256), 0, s, true, m->ws, splits,
+               (size_t)kIn * kHid, m->grad + clsph_nn::kOffW1);
+  launch_early(clsph_nn::k_colsum, dim3(rows / 256), dim3(kHid), 0, s, true, m->dz1, rows, 256,
+               m->grad + clsph_nn::kOffB1);
   return 0;
 }
 
@@ -906,8 +918,7 @@ int clsph_mlp_gradients(clsph_mlp* m, const float* x_raw, const float* y_raw, ui
   int rc;
   if ((rc = ensure_training(m, rows)) || (rc = ensure_loss(m, 1))) return rc;
   CUDA_TRY(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-  clsph_nn::k_gather_batch<<<(rows * (kIn + kOut) + 255) / 256, 256, 0, m->stream>>>(
-      x_raw, y_raw, nullptr, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
+  gather_batch(m, x_raw, y_raw, nullptr, rows, true);
   if ((rc = pass(m, rows, m->loss, true))) return rc;
   float l = 0.f;
   CUDA_TRY(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -928,8 +939,7 @@ int clsph_mlp_loss(clsph_mlp* m, const float* x_raw, const float* y_raw, uint64_
   if ((rc = ensure_training(m, rows)) || (rc = ensure_loss(m, 1))) return rc;
   CUDA_TRY(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
   for (uint64_t b = 0; b < blocks; ++b) {
-    clsph_nn::k_gather_batch<<<(rows * (kIn + kOut) + 255) / 256, 256, 0, m->stream>>>(
-        x_raw + b * rows * kIn, y_raw + b * rows * kOut, nullptr, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
+    gather_batch(m, x_raw + b * rows * kIn, y_raw + b * rows * kOut, nullptr, rows, false);
     if ((rc = pass(m, rows, m->loss, false))) return rc;
   }
   float l = 0.f;
@@ -989,16 +999,16 @@ int clsph_mlp_train(clsph_mlp* m, const float* x_raw, const float* y_raw, uint64
     CUDA_TRY(cudaStreamSynchronize(s));  // the previous epoch's gathers read m->idx
     CUDA_TRY(cudaMemcpyAsync(m->idx, perm.data(), sizeof(uint32_t) * samples, cudaMemcpyHostToDevice, s));
     for (uint64_t b = 0; b < per_epoch; ++b, ++step) {
-      clsph_nn::k_gather_batch<<<(rows * (kIn + kOut) + 255) / 256, 256, 0, s>>>(
-          x_raw, y_raw, m->idx + b * rows, rows, m->blob + clsph_nn::kOffXMu, m->xb, m->yb);
+      gather_batch(m, x_raw, y_raw, m->idx + b * rows, rows, true);
       if ((rc = pass(m, rows, m->loss + step, true))) return rc;
       const float frac = total > 1 ? (float)step / (float)(total - 1) : 0.f;
       const float lr = cfg->lr + (cfg->lr_final - cfg->lr) * frac;
       ++m->adam_t;
       const float bc1 = 1.f - std::pow(beta1, (float)m->adam_t);
       const float bc2 = 1.f - std::pow(beta2, (float)m->adam_t);
-      clsph_nn::k_adam<<<(kParams + 255) / 256, 256, 0, s>>>(m->blob, m->grad, m->adam_m, m->adam_v, kParams,
-                                                            lr, beta1, beta2, eps, bc1, bc2, bf16_weights(m));
+      launch_early(clsph_nn::k_adam, dim3((kParams + 255) / 256), dim3(256), 0, s, true, m->blob,
+                   (const float*)m->grad, m->adam_m, m->adam_v, kParams, lr, beta1, beta2, eps, bc1, bc2,
+                   bf16_weights(m));
     }
   }
   CUDA_TRY(cudaGetLastError());

@@ -23,6 +23,8 @@
 
 #include <cstdint>
 
+#include "clsph_common.cuh"
+
 namespace clsph_nn {
 
 constexpr int kIn = 32;
@@ -384,12 +386,17 @@ struct EpiPartialT {
 // ---------------------------------------------------------------------------
 // Training: elementwise and reduction kernels
 
-// Batch rows from the sample set: x standardised to bf16, y standardised fp32.
+// Batch rows from the sample set: x standardised to bf16, y standardised fp32;
+// clears the gradients that the pass adds to (`grad`, null without a backward
+// pass).
 __global__ void k_gather_batch(const float* __restrict__ x_raw, const float* __restrict__ y_raw,
                                const uint32_t* __restrict__ idx /* or null: the rows as they lie */, uint32_t rows,
                                const float* __restrict__ norm /* blob + kOffXMu */,
-                               bf16* __restrict__ xb, float* __restrict__ yb) {
+                               bf16* __restrict__ xb, float* __restrict__ yb, float* __restrict__ grad) {
+  if (clsph::never_after_previous()) return;
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (grad)
+    for (uint32_t q = t; q < (uint32_t)kParams; q += gridDim.x * blockDim.x) grad[q] = 0.f;
   const uint32_t r = t / (kIn + kOut), c = t % (kIn + kOut);
   if (r >= rows) return;
   const size_t s = idx ? idx[r] : r;
@@ -423,6 +430,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32)
     k_head(const bf16* __restrict__ h2, const float* __restrict__ z2, const float* __restrict__ w3,
            const float* __restrict__ b3, const float* __restrict__ yt, uint32_t rows, float inv_rows, bf16* __restrict__ dz2, float* __restrict__ dw3,
            float* __restrict__ db3, float* __restrict__ db2, float* __restrict__ loss_sum) {
+  if (clsph::never_after_previous()) return;
   static_assert(kHid == 256 && kOut == 4, "eight hidden units a lane");
   __shared__ float sw[kHid * kOut];
   __shared__ float sb2[kHid];
@@ -510,6 +518,7 @@ __global__ void __launch_bounds__(kHeadWarps * 32)
 // db[c] += sum over rows of dz[r][c] (bf16 [rows][256]): 32 threads a row, eight columns each
 __global__ void __launch_bounds__(256) k_colsum(const bf16* __restrict__ dz, uint32_t rows, uint32_t rows_per_block,
                                                 float* __restrict__ db) {
+  if (clsph::never_after_previous()) return;
   __shared__ float part[8][kHid];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t r_begin = blockIdx.x * rows_per_block;
@@ -537,6 +546,7 @@ __global__ void __launch_bounds__(256) k_colsum(const bf16* __restrict__ dz, uin
 // out[i] = sum over splits of ws[s][i]
 __global__ void k_reduce_splits(const float* __restrict__ ws, int splits, size_t count,
                                 float* __restrict__ out) {
+  if (clsph::never_after_previous()) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   float s = 0.f;
@@ -579,6 +589,7 @@ struct Bf16Weights {
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ grad, float* __restrict__ m,
                        float* __restrict__ v, int count, float lr, float beta1, float beta2, float eps,
                        float bc1, float bc2, Bf16Weights wb) {
+  if (clsph::never_after_previous()) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float gr = grad[i];

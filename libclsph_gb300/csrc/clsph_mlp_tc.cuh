@@ -489,6 +489,7 @@ template <int BN, bool A_K, bool B_K, class Epi>
 __global__ void __launch_bounds__(kGtThreads, 1)
     k_gemm_tc(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B, int ldb, int K, int k_split,
               Epi epi, uint32_t* __restrict__ err) {
+  if (clsph::never_after_previous()) return;
   using L = GemmTcLayout<BN>;
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t sb = smem_addr(smem);
