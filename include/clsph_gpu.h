@@ -213,7 +213,9 @@ int clsph_gpu_kernel_times(clsph_gpu* h, int max_classes, char* names, int name_
 int clsph_gpu_autotune(clsph_gpu* h, uint32_t substeps, char* report, int report_len);
 
 /* Sets the launch shapes directly (e.g. from a cached autotune result):
- * blocks of 64, 128 or 256 threads; 1..64 advection blocks per SM. */
+ * blocks of 64, 128 or 256 threads; 1..64 advection blocks per SM. (Scenes of
+ * up to 40,000 particles run the forces with several lanes per particle in
+ * blocks of their own size.) */
 int clsph_gpu_set_launch_shape(clsph_gpu* h, int density_block, int forces_block,
                                uint32_t advect_blocks_per_sm);
 
@@ -243,7 +245,7 @@ int clsph_gpu_set_neighbour_search(clsph_gpu* h, int mode);
  * up to 64 substeps per launch, for handles of any number of scenes. The
  * results equal the launched substeps' bit for bit (the same block-level
  * code); clsph_gpu_autotune keeps whichever form is faster. Neighbour search
- * is CELL_WARPS with 8 warps per block; per-kernel profiling and
+ * is CELL_WARPS with teams of two warps; per-kernel profiling and
  * clsph_gpu_step_until launch the kernels as usual. CLSPH_ERR_CUDA if the
  * device has no cooperative launch. */
 int clsph_gpu_set_persistent(clsph_gpu* h, int enabled);
@@ -272,8 +274,8 @@ int clsph_gpu_read_face_lists(clsph_gpu* h, uint32_t scene, float* plan, uint32_
 
 /* Bounds of the engine's device-side waits; no counterpart in the reference,
  * whose OpenCL queue has no device-side waits. radix_lookback_spins bounds
- * each radix-sort look-back wait (default CLSPH_DEFAULT_LOOKBACK_SPINS): a
- * wait that runs out leaves that substep's order wrong, keeps every access in
+ * each radix-sort wait, for a tile's look-back words and for the pass before
+ * (default CLSPH_DEFAULT_LOOKBACK_SPINS): a wait that runs out leaves that substep's order wrong, keeps every access in
  * bounds and makes the next clsph_gpu_sync return CLSPH_ERR_CUDA.
  * mlp_wait_polls bounds each mbarrier wait of the learned stepper's tcgen05
  * MLP kernel (default CLSPH_DEFAULT_MLP_WAIT_POLLS; 0 gives up at once): a wait

@@ -962,10 +962,10 @@ static __global__ void __launch_bounds__(kParticleWarps * 32)
 //
 // Bound: instruction issue, half of it the exact evaluation. 1,048,576
 // particles spread over a floor (29,552 cells, a quarter of them of one or
-// two particles): 212 M warp instructions, 60 % of the issue slots, 0.309 ms,
+// two particles): 212 M warp instructions, 60 % of the issue slots, 0.303 ms,
 // against 313 M and 0.454 ms for the form before, one warp per cell that
 // tested each of its 64 particles against all 512 candidates in FP32; the
-// same on the h/2 lattice: 0.235 ms against 0.359. Of the 212 M: the cell's
+// same on the h/2 lattice: 0.230 ms against 0.359. Of the 212 M: the cell's
 // look-up and the outputs 38 M, candidates 24 M, culls 38 M (an octant's 216
 // candidates instead of 512, two per operation), exact evaluation 112 M.
 // Staging with FP32 positions streamed per neighbour list and compacted by

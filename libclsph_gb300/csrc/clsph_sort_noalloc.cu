@@ -23,6 +23,11 @@
 //    cudaGetSymbolAddress (with that device current); make that first call
 //    before any stream capture.
 // It makes no cudaMalloc, cudaFree or other allocating call.
+//
+// Bound: the sort's own latencies (clsph_radix.cuh). Three launches, each with
+// its blocks placed while the one before still runs: 1,048,576 keys of 22 bits
+// 35 us, against 46 with a memset node and plain launches (39 with the memset
+// kept) and 91 with a launch per pass and step.
 
 #include <cuda_runtime.h>
 
