@@ -219,7 +219,10 @@ __device__ __forceinline__ void grid_setup_block(uint32_t* __restrict__ bbox_all
   g.half_margin = (float)(gmax + 2) * 0x1p-20f;
   for (int i = 0; i < 4; ++i) g.pad_[i] = 0u;
   *grid = g;
-  if (overflow) atomicOr(status, kFlagGridOverflow);
+  if (overflow) {  // (flagged) cells holds the wrapped sizes, and coordinates wrap at ten bits: take all the bits there are
+    atomicOr(status, kFlagGridOverflow);
+    atomicMax(&shift_s, min(30u, 32u - ctl[kCtlSceneBits]));
+  }
   // sentinels of sph_simulation.cpp:204-205 for the next accumulation
   for (int a = 0; a < 3; ++a) {
     bbox[a] = f2ord(2147483648.0f);
@@ -407,7 +410,8 @@ __device__ __forceinline__ void keys_blocks(uint32_t blk, uint32_t nblk, const f
                                             uint32_t ntiles, uint4* __restrict__ index_keys, uint32_t index_quads,
                                             KeysSmem& sm) {
   const KeySplit split{ctl[kCtlShift]};
-  // no key has more bits than the widest grid's keys and the scenes
+  // no key has more bits than the widest grid's keys and the scenes (the Morton part is masked: on an overflowed
+  // grid it can hold more)
   const uint32_t passes = (min(split.shift + ctl[kCtlSceneBits], 32u) + 7u) / 8u;
   const uint32_t first = blk * blockDim.x + threadIdx.x, stride = nblk * blockDim.x;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -426,7 +430,7 @@ __device__ __forceinline__ void keys_blocks(uint32_t blk, uint32_t nblk, const f
       const uint32_t cx = __float2uint_rz(XDIV(XSUB(p.x, g.lo[0]), g.cell));
       const uint32_t cy = __float2uint_rz(XDIV(XSUB(p.y, g.lo[1]), g.cell));
       const uint32_t cz = __float2uint_rz(XDIV(XSUB(p.z, g.lo[2]), g.cell));
-      key = morton3(cx, cy, cz) | split.scene_bits(sc);
+      key = split.morton(morton3(cx, cy, cz)) | split.scene_bits(sc);
       keys[i] = key;
       top = max(top, key);
     }
@@ -1078,6 +1082,7 @@ __device__ __forceinline__ void density_cells_team(
   if (wid == 0 && lane < 4u) sm.no_chunk[lane] = make_uint4(0u, 0u, 0u, kNever * 0x10001u);
   const uint32_t ncells = counters[kCntCells];
   const KeySplit split{ctl[kCtlShift]};
+  const bool whole_keys = split.shift + ctl[kCtlSceneBits] <= 32u;  // (if not, flagged, keys lose upper scene bits)
   auto by_warp = [&](uint32_t i) {
     density_particle_warp(i, n, grids, scene_of, split, keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n, pos, ci,
                           consts, aux_out, nlist, ncount, nlist_cap, vel, frec, nb_start);
@@ -1119,7 +1124,7 @@ __device__ __forceinline__ void density_cells_team(
       const uint32_t own_e = __shfl_sync(0xFFFFFFFFu, e, 13);
       const uint32_t count = own_e > own.x ? own_e - own.x : 0u;
       uint32_t candidates = kNoLists;
-      const uint32_t sc = split.shift >= 32u ? 0u : own.y >> split.shift;
+      const uint32_t sc = whole_keys ? (split.shift >= 32u ? 0u : own.y >> split.shift) : scene_of[own.x];
       if (!__any_sync(0xFFFFFFFFu, e - s >= (1u << kCellOffBits)) && count > kSparseCell && consts[sc].plain_h) {
         // the candidates of list k as bits, in up to three words of the planes (more are counted and read again)
         const uint32_t need = kOffsetMasks.m[min(lane, 26u)];
