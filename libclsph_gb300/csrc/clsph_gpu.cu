@@ -441,9 +441,15 @@ int build_face_lists(clsph_gpu* h, SceneMesh& sm, uint32_t faces, const FaceGrid
   return done(0);
 }
 
+// (Copies to the device and clears go through the stream of the kernels that
+// read them: a cudaMemcpy from pageable memory may return before its last piece
+// has arrived, and the handle's own stream does not wait for the default one.)
 int sync_scene_tables(clsph_gpu* h) {
-  CUDA_TRY(cudaMemcpy(h->consts, h->consts_host.data(), sizeof(Consts) * h->nscenes, cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(h->meshes, h->mesh_host.data(), sizeof(DevMesh) * h->nscenes, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpyAsync(h->consts, h->consts_host.data(), sizeof(Consts) * h->nscenes, cudaMemcpyHostToDevice,
+                           h->stream));
+  CUDA_TRY(cudaMemcpyAsync(h->meshes, h->mesh_host.data(), sizeof(DevMesh) * h->nscenes, cudaMemcpyHostToDevice,
+                           h->stream));
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
   return 0;
 }
 
@@ -540,19 +546,20 @@ int clsph_gpu_create_batched(const clsph_parameters* params, const clsph_kernel_
   }
   std::vector<uint32_t> iota(n);
   for (uint32_t i = 0; i < n; ++i) iota[i] = i;
-  if (cudaMemset(h->grids, 0, sizeof(DevGrid) * nscenes) != cudaSuccess ||
-      cudaMemset(h->status, 0, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMemset(h->pbar, 0, 2 * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMemset(h->capped, 0, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemset(h->aux, 0, sizeof(float4) * n) != cudaSuccess ||
-      cudaMemset(h->ncount, 0, sizeof(uint32_t) * n) != cudaSuccess ||
-      cudaMemset(h->keys, 0, sizeof(uint32_t) * 2 * (size_t)n) != cudaSuccess ||
-      cudaMemset(h->vals, 0, sizeof(uint32_t) * 2 * (size_t)n) != cudaSuccess ||
-      cudaMemset(h->acc, 0, sizeof(float4) * n) != cudaSuccess ||
-      cudaMemcpy(h->ctl, ctl_init, sizeof(ctl_init), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(h->scene_of, scene_of.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(h->scene_h, hs.data(), sizeof(float) * nscenes, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(h->ids[0], iota.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
+  if (cudaMemsetAsync(h->grids, 0, sizeof(DevGrid) * nscenes, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->status, 0, sizeof(uint32_t), h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->pbar, 0, 2 * sizeof(uint32_t), h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->capped, 0, sizeof(unsigned long long), h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->aux, 0, sizeof(float4) * n, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->ncount, 0, sizeof(uint32_t) * n, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->keys, 0, sizeof(uint32_t) * 2 * (size_t)n, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->vals, 0, sizeof(uint32_t) * 2 * (size_t)n, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(h->acc, 0, sizeof(float4) * n, h->stream) != cudaSuccess ||
+      cudaMemcpyAsync(h->ctl, ctl_init, sizeof(ctl_init), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+      cudaMemcpyAsync(h->scene_of, scene_of.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice, h->stream) !=
+          cudaSuccess ||
+      cudaMemcpyAsync(h->scene_h, hs.data(), sizeof(float) * nscenes, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+      cudaMemcpyAsync(h->ids[0], iota.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
     return bail(fail(CLSPH_ERR_CUDA, "create: initialisation copies"));
   if ((rc = sync_scene_tables(h))) return bail(rc);
   *out = h;
@@ -635,9 +642,9 @@ int clsph_gpu_set_scene_mesh(clsph_gpu* h, uint32_t scene, const float* normals,
         (rc = dev_alloc(&sm.indices, 3 * (size_t)faces)) ||
         (rc = dev_alloc(&sm.packed, kFaceRows * (size_t)faces)))
       return rc;
-    CUDA_TRY(cudaMemcpy(sm.normals, normals, sizeof(float) * 3 * faces, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(sm.vertices, vertices, sizeof(float) * 3 * vertex_count, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(sm.indices, indices, sizeof(uint32_t) * 3 * faces, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(sm.normals, normals, sizeof(float) * 3 * faces, cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(cudaMemcpyAsync(sm.vertices, vertices, sizeof(float) * 3 * vertex_count, cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(cudaMemcpyAsync(sm.indices, indices, sizeof(uint32_t) * 3 * faces, cudaMemcpyHostToDevice, h->stream));
     k_pack_faces<<<grid_blocks(faces, h->sm_count * 8), kBlock, 0, h->stream>>>(sm.normals, sm.vertices, sm.indices,
                                                                                 faces, sm.packed);
     CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -795,10 +802,10 @@ int clsph_gpu_sync(clsph_gpu* h, uint32_t* flags) {
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   uint32_t f = 0;
   CUDA_TRY(cudaMemcpy(&f, h->status, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-  CUDA_TRY(cudaMemset(h->status, 0, sizeof(uint32_t)));
+  CUDA_TRY(cudaMemsetAsync(h->status, 0, sizeof(uint32_t), h->stream));
   if (f & kFlagBarrierStall) {
     // the barrier words may be left mid-count: start the next launch afresh
-    CUDA_TRY(cudaMemset(h->pbar, 0, 2 * sizeof(uint32_t)));
+    CUDA_TRY(cudaMemsetAsync(h->pbar, 0, 2 * sizeof(uint32_t), h->stream));
     return fail(CLSPH_ERR_CUDA, "sync: a grid barrier wait of the persistent substep kernel ran out "
                                 "(the substeps of that launch are incomplete)");
   }
@@ -832,7 +839,7 @@ int clsph_gpu_set_scene_parameters(clsph_gpu* h, uint32_t scene, const clsph_par
   h->terms[scene] = *terms;
   h->consts_host[scene] = derive_consts(p, *terms, count);
   const float hs = p.h;
-  CUDA_TRY(cudaMemcpy(h->scene_h + scene, &hs, sizeof(float), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpyAsync(h->scene_h + scene, &hs, sizeof(float), cudaMemcpyHostToDevice, h->stream));
   return sync_scene_tables(h);
 }
 

@@ -410,7 +410,7 @@ int check_train_waits(clsph_mlp* m) {
   CUDA_TRY(cudaMemcpy(&e, m->err, sizeof(e), cudaMemcpyDeviceToHost));
   if (e & kTrainWaitBit) {
     const uint32_t keep = e & ~kTrainWaitBit;
-    CUDA_TRY(cudaMemcpy(m->err, &keep, sizeof(keep), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(m->err, &keep, sizeof(keep), cudaMemcpyHostToDevice, m->stream));
     return fail(CLSPH_ERR_CUDA, "mlp: a tensor-core wait of a training GEMM timed out");
   }
   return 0;
@@ -429,8 +429,8 @@ int ensure_training(clsph_mlp* m, uint32_t rows) {
     if ((rc = alloc(&m->grad, kParams)) || (rc = alloc(&m->adam_m, kParams)) ||
         (rc = alloc(&m->adam_v, kParams)) || (rc = alloc(&m->moments, 2 * (kIn + kOut))))
       return rc;
-    CUDA_TRY(cudaMemset(m->adam_m, 0, sizeof(float) * kParams));
-    CUDA_TRY(cudaMemset(m->adam_v, 0, sizeof(float) * kParams));
+    CUDA_TRY(cudaMemsetAsync(m->adam_m, 0, sizeof(float) * kParams, m->stream));
+    CUDA_TRY(cudaMemsetAsync(m->adam_v, 0, sizeof(float) * kParams, m->stream));
     m->adam_t = 0;
   }
   if (rows > m->rows_cap) {
@@ -607,9 +607,9 @@ int ensure_cache(clsph_gpu* h, LearnedCache** out) {
       return bail(rc);
   // the correction and feature rows start defined: a learned step whose MLP
   // stopped early (a wait ran out, reported as an error) reads them as they are
-  if (cudaMemset(L->dev_sum, 0, (kGateSums + 1) * sizeof(float)) != cudaSuccess ||
-      cudaMemset(L->corr, 0, sizeof(float4) * n) != cudaSuccess ||
-      cudaMemset(L->x, 0, sizeof(bf16) * n * kFeat) != cudaSuccess ||
+  if (cudaMemsetAsync(L->dev_sum, 0, (kGateSums + 1) * sizeof(float), h->stream) != cudaSuccess ||
+      cudaMemsetAsync(L->corr, 0, sizeof(float4) * n, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(L->x, 0, sizeof(bf16) * n * kFeat, h->stream) != cudaSuccess ||
       cudaMallocHost(reinterpret_cast<void**>(&L->dev_host), (kGateSums + 1) * sizeof(float)) != cudaSuccess ||
       cudaEventCreateWithFlags(&L->ev, cudaEventDisableTiming) != cudaSuccess)
     return bail(fail(CLSPH_ERR_CUDA, "step_learned: buffer set-up"));
@@ -815,7 +815,8 @@ int clsph_mlp_create(uint64_t seed, clsph_mlp** out) {
       (rc = alloc(&m->w3b, kHid * kOutPad)) || (rc = alloc(&m->w1t, kIn * kHid)) ||
       (rc = alloc(&m->w2t, kHid * kHid)) || (rc = alloc(&m->w3t, 16 * kHid)) || (rc = alloc(&m->err, 1)))
     return bail(rc);
-  if (cudaMemset(m->err, 0, sizeof(uint32_t)) != cudaSuccess) return bail(fail(CLSPH_ERR_CUDA, "mlp_create: memset"));
+  if (cudaMemsetAsync(m->err, 0, sizeof(uint32_t), m->stream) != cudaSuccess)
+    return bail(fail(CLSPH_ERR_CUDA, "mlp_create: memset"));
   std::vector<float> blob(kBlob, 0.f);
   std::mt19937_64 rng(seed);
   std::normal_distribution<float> nd(0.f, 1.f);
@@ -825,7 +826,7 @@ int clsph_mlp_create(uint64_t seed, clsph_mlp** out) {
   for (int i = 0; i < kHid * kOut; ++i) blob[clsph_nn::kOffW3 + i] = nd(rng) * s3;
   for (int i = 0; i < kIn; ++i) blob[clsph_nn::kOffXSigma + i] = 1.f;
   for (int i = 0; i < kOut; ++i) blob[clsph_nn::kOffYSigma + i] = 1.f;
-  if (cudaMemcpy(m->blob, blob.data(), sizeof(float) * kBlob, cudaMemcpyHostToDevice) != cudaSuccess)
+  if (cudaMemcpyAsync(m->blob, blob.data(), sizeof(float) * kBlob, cudaMemcpyHostToDevice, m->stream) != cudaSuccess)
     return bail(fail(CLSPH_ERR_CUDA, "mlp_create: upload"));
   if ((rc = refresh_bf16(m)) || cudaStreamSynchronize(m->stream) != cudaSuccess)
     return bail(rc ? rc : fail(CLSPH_ERR_CUDA, "mlp_create: weight conversion"));
@@ -838,14 +839,14 @@ int clsph_mlp_set_blob(clsph_mlp* m, const float* blob, uint64_t count) {
   for (int i = 0; i < kIn; ++i)
     if (!(blob[clsph_nn::kOffXSigma + i] > 0.f)) return fail(CLSPH_ERR_ARGUMENT, "mlp_set_blob: x_sigma <= 0");
   CUDA_TRY(cudaStreamSynchronize(m->stream));
-  CUDA_TRY(cudaMemcpy(m->blob, blob, sizeof(float) * kBlob, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpyAsync(m->blob, blob, sizeof(float) * kBlob, cudaMemcpyHostToDevice, m->stream));
   int rc = refresh_bf16(m);
   if (rc) return rc;
   CUDA_TRY(cudaStreamSynchronize(m->stream));
   m->adam_t = 0;
   if (m->adam_m) {
-    CUDA_TRY(cudaMemset(m->adam_m, 0, sizeof(float) * kParams));
-    CUDA_TRY(cudaMemset(m->adam_v, 0, sizeof(float) * kParams));
+    CUDA_TRY(cudaMemsetAsync(m->adam_m, 0, sizeof(float) * kParams, m->stream));
+    CUDA_TRY(cudaMemsetAsync(m->adam_v, 0, sizeof(float) * kParams, m->stream));
   }
   return CLSPH_OK;
 }
@@ -907,7 +908,7 @@ int clsph_mlp_status(clsph_mlp* m, uint32_t* flags) {
   if (!m || !flags) return fail(CLSPH_ERR_ARGUMENT, "mlp_status: bad argument");
   CUDA_TRY(cudaDeviceSynchronize());
   CUDA_TRY(cudaMemcpy(flags, m->err, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-  CUDA_TRY(cudaMemset(m->err, 0, sizeof(uint32_t)));
+  CUDA_TRY(cudaMemsetAsync(m->err, 0, sizeof(uint32_t), m->stream));
   return CLSPH_OK;
 }
 
@@ -1062,8 +1063,8 @@ int clsph_collector_create(clsph_gpu* h, uint32_t id_stride, uint32_t dt_mult, u
     clsph_collector_destroy(c);
     return rc;
   }
-  if (cudaMemset(c->zero, 0, sizeof(float4) * n) != cudaSuccess ||
-      cudaMemset(c->sbbox, 0, sizeof(uint32_t) * 6 * h->nscenes) != cudaSuccess) {
+  if (cudaMemsetAsync(c->zero, 0, sizeof(float4) * n, h->stream) != cudaSuccess ||
+      cudaMemsetAsync(c->sbbox, 0, sizeof(uint32_t) * 6 * h->nscenes, h->stream) != cudaSuccess) {
     clsph_collector_destroy(c);
     return fail(CLSPH_ERR_CUDA, "collector_create: memset");
   }
