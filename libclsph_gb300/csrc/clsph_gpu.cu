@@ -441,6 +441,43 @@ int build_face_lists(clsph_gpu* h, SceneMesh& sm, uint32_t faces, const FaceGrid
   return done(0);
 }
 
+// Uploads a mesh of at least one face into the scene's (empty) slots.
+int upload_mesh(clsph_gpu* h, uint32_t scene, const float* normals, const float* vertices, uint32_t vertex_count,
+                const uint32_t* indices, uint32_t faces) {
+  SceneMesh& sm = h->scene_mesh[scene];
+  DevMesh& dm = h->mesh_host[scene];
+  int rc;
+  if ((rc = dev_alloc(&sm.normals, 3 * (size_t)faces)) ||
+      (rc = dev_alloc(&sm.vertices, 3 * (size_t)vertex_count)) ||
+      (rc = dev_alloc(&sm.indices, 3 * (size_t)faces)) ||
+      (rc = dev_alloc(&sm.packed, kFaceRows * (size_t)faces)))
+    return rc;
+  CUDA_TRY(cudaMemcpyAsync(sm.normals, normals, sizeof(float) * 3 * faces, cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(cudaMemcpyAsync(sm.vertices, vertices, sizeof(float) * 3 * vertex_count, cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(cudaMemcpyAsync(sm.indices, indices, sizeof(uint32_t) * 3 * faces, cudaMemcpyHostToDevice, h->stream));
+  k_pack_faces<<<grid_blocks(faces, h->sm_count * 8), kBlock, 0, h->stream>>>(sm.normals, sm.vertices, sm.indices,
+                                                                              faces, sm.packed);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
+  dm.packed = sm.packed;
+  dm.faces = faces;
+  FaceGridPlan plan{};
+  float reach = 0.f;
+  rc = plan_face_grid(h->params[scene], vertices, vertex_count, indices, faces, plan, reach);
+  if (rc >= 256) return rc;
+  if (rc) return 0;  // (a non-finite mesh keeps no lists: every face is scanned)
+  if ((rc = build_face_lists(h, sm, faces, plan))) return rc;
+  dm.cell_start = sm.cell_start;
+  dm.cell_faces = sm.cell_faces;
+  for (int a = 0; a < 3; ++a) {
+    dm.lo[a] = plan.glo[a];
+    dm.dims[a] = plan.dims[a];
+  }
+  dm.inv_cell = 1.f / plan.cell;
+  dm.reach = reach;
+  return 0;
+}
+
 // (Copies to the device and clears go through the stream of the kernels that
 // read them: a cudaMemcpy from pageable memory may return before its last piece
 // has arrived, and the handle's own stream does not wait for the default one.)
@@ -631,42 +668,15 @@ int clsph_gpu_set_scene_mesh(clsph_gpu* h, uint32_t scene, const float* normals,
   for (uint64_t k = 0; k < 3ull * faces; ++k)
     if (indices[k] >= vertex_count) return fail(CLSPH_ERR_ARGUMENT, "set_mesh: vertex index out of range");
   CUDA_TRY(cudaStreamSynchronize(h->stream));
-  SceneMesh& sm = h->scene_mesh[scene];
-  DevMesh& dm = h->mesh_host[scene];
-  sm.release();
-  dm = DevMesh{};
-  if (faces) {
-    int rc;
-    if ((rc = dev_alloc(&sm.normals, 3 * (size_t)faces)) ||
-        (rc = dev_alloc(&sm.vertices, 3 * (size_t)vertex_count)) ||
-        (rc = dev_alloc(&sm.indices, 3 * (size_t)faces)) ||
-        (rc = dev_alloc(&sm.packed, kFaceRows * (size_t)faces)))
-      return rc;
-    CUDA_TRY(cudaMemcpyAsync(sm.normals, normals, sizeof(float) * 3 * faces, cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(sm.vertices, vertices, sizeof(float) * 3 * vertex_count, cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(sm.indices, indices, sizeof(uint32_t) * 3 * faces, cudaMemcpyHostToDevice, h->stream));
-    k_pack_faces<<<grid_blocks(faces, h->sm_count * 8), kBlock, 0, h->stream>>>(sm.normals, sm.vertices, sm.indices,
-                                                                                faces, sm.packed);
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
-    dm.packed = sm.packed;
-    dm.faces = faces;
-    FaceGridPlan plan{};
-    float reach = 0.f;
-    rc = plan_face_grid(h->params[scene], vertices, vertex_count, indices, faces, plan, reach);
-    if (rc >= 256) return rc;
-    if (rc == 0) {  // (a non-finite mesh keeps no lists: every face is scanned)
-      if ((rc = build_face_lists(h, sm, faces, plan))) return rc;
-      dm.cell_start = sm.cell_start;
-      dm.cell_faces = sm.cell_faces;
-      for (int a = 0; a < 3; ++a) {
-        dm.lo[a] = plan.glo[a];
-        dm.dims[a] = plan.dims[a];
-      }
-      dm.inv_cell = 1.f / plan.cell;
-      dm.reach = reach;
-    }
+  h->scene_mesh[scene].release();
+  h->mesh_host[scene] = DevMesh{};
+  const int rc = faces ? upload_mesh(h, scene, normals, vertices, vertex_count, indices, faces) : 0;
+  if (rc) {  // the scene has no mesh then; its table entry must not keep the freed one's pointers
+    h->scene_mesh[scene].release();
+    h->mesh_host[scene] = DevMesh{};
   }
-  return sync_scene_tables(h);
+  const int table = sync_scene_tables(h);
+  return rc ? rc : table;
 }
 
 int clsph_gpu_read_face_lists(clsph_gpu* h, uint32_t scene, float* plan, uint32_t* cell_start,
