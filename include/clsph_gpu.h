@@ -311,9 +311,18 @@ int clsph_gpu_counters(clsph_gpu* h, uint64_t* out3);
  * the life of the process: after cudaDeviceReset the device's code is loaded
  * anew and that address is stale, so a process that resets a device must not
  * call this function on it again. Asynchronous on
- * `cuda_stream` (a cudaStream_t, NULL = legacy default stream). */
+ * `cuda_stream` (a cudaStream_t, NULL = legacy default stream). The sort's
+ * blocks wait for one another, each wait bounded by
+ * CLSPH_DEFAULT_LOOKBACK_SPINS; should one run out, a single block sorts
+ * everything again without waits: the outputs are the same, some
+ * milliseconds later for 1,048,576 keys. */
 int clsph_gpu_sort_keys_noalloc(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* perm_out,
                                 uint32_t n, void* cuda_stream);
+/* The same with the waits' bound given and, for tests, one tile of every pass
+ * (CLSPH_NO_TILE: none) that withholds its digit counts. */
+int clsph_gpu_sort_keys_noalloc_limited(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* perm_out, uint32_t n,
+                                        void* cuda_stream, uint32_t radix_lookback_spins,
+                                        uint32_t radix_withheld_tile);
 
 /* Text of the last error on this thread. */
 const char* clsph_gpu_last_error(void);

@@ -17,7 +17,8 @@
 // that is already running and whose own waits are for earlier tickets; every
 // wait is bounded all the same (spin_limit, by default kRadixLookbackSpins),
 // and one that runs out raises kFlagSortStall, which clsph_gpu_sync reports as
-// an error. After a stall the offsets of the tiles behind it are wrong, but
+// an error (the stand-alone sort, which has no later call to report it, sorts
+// again in one block). After a stall the offsets of the tiles behind it are wrong, but
 // every store stays in bounds (destinations >= n are skipped, and the slots a
 // pass leaves unwritten keep earlier in-range values), so the context stays
 // usable.
@@ -116,8 +117,10 @@ struct RadixSmem {
 };
 
 // Every pass, by all blocks of the grid: `counters` are the ticket and the
-// tiles done of each pass (zero at the start, as the look-back words).
-template <uint32_t THREADS>
+// tiles done of each pass (zero at the start, as the look-back words). kAlone:
+// by the calling block alone, tile after tile, with the digits' counts of the
+// tiles before carried from tile to tile and no waits.
+template <uint32_t THREADS, bool kAlone = false>
 __device__ __forceinline__ void radix_sort_blocks(const RadixBuffers& buf, uint32_t n, uint32_t passes,
                                                   const uint32_t* __restrict__ digit_total,
                                                   uint32_t* __restrict__ lookback, uint32_t ntiles,
@@ -127,9 +130,12 @@ __device__ __forceinline__ void radix_sort_blocks(const RadixBuffers& buf, uint3
   constexpr uint32_t kWarps = THREADS / 32, kItems = kRadixTile / THREADS, kSpan = 32 * kItems;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, d = threadIdx.x;
   const uint32_t lt_mask = (1u << lane) - 1u;
+  uint32_t turn = 0, carry = 0;
   for (;;) {
     __syncthreads();  // the block's previous tile is done with the shared arrays
-    if (threadIdx.x == 0) {
+    if (kAlone) {
+      if (threadIdx.x == 0) sm.ticket = turn++;
+    } else if (threadIdx.x == 0) {
       const uint32_t t = atomicAdd(&counters[0], 1u);
       const uint32_t p = t / ntiles;
       if (p > 0u && p < passes) {
@@ -187,7 +193,7 @@ __device__ __forceinline__ void radix_sort_blocks(const RadixBuffers& buf, uint3
         local += c;
       }
       uint32_t* lb = lookback + (size_t)pass * ntiles * 256u + d;
-      const bool publish = tile != withheld_tile;
+      const bool publish = !kAlone && tile != withheld_tile;
       if (publish) st_relaxed_gpu(&lb[(size_t)tile * 256u], (tile == 0 ? kLbInclusive : kLbAggregate) | local);
       // keys with a smaller digit: exclusive scan of the pass's digit totals
       total = digit_total[pass * 256u + d];
@@ -198,7 +204,10 @@ __device__ __forceinline__ void radix_sort_blocks(const RadixBuffers& buf, uint3
         if (lane >= off) below += y;
       }
       if (lane == 31u) sm.warp_sums[warp] = below;
-      if (tile > 0) {
+      if (kAlone) {
+        excl = tile ? carry : 0u;
+        carry = excl + local;
+      } else if (tile > 0) {
         // walk back kWindow tiles per round (independent loads), adding published counts until an inclusive
         // prefix (tile 0 always has one)
         constexpr int kWindow = 8;
@@ -247,7 +256,7 @@ __device__ __forceinline__ void radix_sort_blocks(const RadixBuffers& buf, uint3
       vals_out[dst] = val[r];
     }
     __syncthreads();
-    if (threadIdx.x == 0 && pass + 1u < passes) {
+    if (!kAlone && threadIdx.x == 0 && pass + 1u < passes) {
       __threadfence();  // the block's stores (ordered by the barrier above) before the count
       atomicAdd(&counters[pass + 1u], 1u);
     }

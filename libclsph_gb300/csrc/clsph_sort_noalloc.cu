@@ -24,10 +24,11 @@
 //    before any stream capture.
 // It makes no cudaMalloc, cudaFree or other allocating call.
 //
-// Bound: the sort's own latencies (clsph_radix.cuh). Three launches, each with
+// Bound: the sort's own latencies (clsph_radix.cuh). Four launches, each with
 // its blocks placed while the one before still runs: 1,048,576 keys of 22 bits
-// 35 us, against 46 with a memset node and plain launches (39 with the memset
-// kept) and 91 with a launch per pass and step.
+// 37 us, against 91 with a launch per pass and step. Without the last launch,
+// which is there for a wait that ran out, 35; without it and with a memset node
+// and plain launches 46 (39 with the memset alone).
 
 #include <cuda_runtime.h>
 
@@ -91,16 +92,40 @@ __global__ void __launch_bounds__(kThreads) k_na_count(const uint32_t* __restric
 }
 
 // The last pass always lands in the caller's output.
+__device__ __forceinline__ RadixBuffers caller_buffers(const uint32_t* keys, uint32_t* keys_out, uint32_t* vals_out,
+                                                       uint32_t passes, uint32_t* scratch) {
+  return RadixBuffers{keys, scratch + kOffKeys, keys_out, scratch + kOffVals, vals_out, (passes + 1u) & 1u};
+}
+
 __global__ void __launch_bounds__(kRadixThreads)
     k_na_sort(const uint32_t* __restrict__ keys, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-              uint32_t n, uint32_t ntiles, uint32_t* __restrict__ scratch) {
+              uint32_t n, uint32_t ntiles, uint32_t* __restrict__ scratch, uint32_t spin_limit,
+              uint32_t withheld_tile) {
   if (never_after_previous()) return;
   __shared__ RadixSmem<kRadixThreads> sm;
   uint32_t* ctl = scratch + kOffCtl;
   const uint32_t passes = radix_passes(ctl[kMaxKey]);
-  const RadixBuffers buf{keys, scratch + kOffKeys, keys_out, scratch + kOffVals, vals_out, (passes + 1u) & 1u};
+  const RadixBuffers buf = caller_buffers(keys, keys_out, vals_out, passes, scratch);
   radix_sort_blocks<kRadixThreads>(buf, n, passes, scratch + kOffTotals, scratch + kOffLookback, ntiles,
-                                   ctl + kCounters, ctl + kStatus, kRadixLookbackSpins, kNoTile, sm);
+                                   ctl + kCounters, ctl + kStatus, spin_limit, withheld_tile, sm);
+}
+
+// The call has returned by now, so a wait that ran out cannot be reported: one
+// block sorts everything again without waits (the input is untouched, and the
+// digit counts do not depend on the order). 6.7 ms for 1,048,576 keys of 22
+// bits; without a stall the launch adds 1.4 us. (In the sort kernel itself,
+// by its last block to finish, the count of blocks alone took 2 us.)
+__global__ void __launch_bounds__(kRadixThreads)
+    k_na_again(const uint32_t* __restrict__ keys, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+               uint32_t n, uint32_t ntiles, uint32_t* __restrict__ scratch) {
+  if (never_after_previous()) return;
+  uint32_t* ctl = scratch + kOffCtl;
+  if (ctl[kStatus] == 0u) return;
+  __shared__ RadixSmem<kRadixThreads> sm;
+  const uint32_t passes = radix_passes(ctl[kMaxKey]);
+  const RadixBuffers buf = caller_buffers(keys, keys_out, vals_out, passes, scratch);
+  radix_sort_blocks<kRadixThreads, true>(buf, n, passes, scratch + kOffTotals, scratch + kOffLookback, ntiles,
+                                         ctl + kCounters, ctl + kStatus, 0u, kNoTile, sm);
 }
 
 // Device address of g_sort_scratch, looked up once per device and kept for
@@ -139,8 +164,9 @@ int scratch_for_current_device(uint32_t** out) {
 
 }  // namespace
 
-extern "C" int clsph_gpu_sort_keys_noalloc(const uint32_t* keys_in, uint32_t* keys_out,
-                                           uint32_t* perm_out, uint32_t n, void* stream) {
+extern "C" int clsph_gpu_sort_keys_noalloc_limited(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* perm_out,
+                                                   uint32_t n, void* stream, uint32_t spin_limit,
+                                                   uint32_t withheld_tile) {
   if (n > kNoAllocMaxKeys) {
     clsph_set_last_error("sort_keys_noalloc: n = " + std::to_string(n) +
                          " exceeds the maximum of 1048576 keys");
@@ -161,11 +187,17 @@ extern "C" int clsph_gpu_sort_keys_noalloc(const uint32_t* keys_in, uint32_t* ke
   launch_early(k_na_count, dim3(blocks < 608u ? blocks : 608u), dim3(kThreads), 0, s, true, keys_in, n, ntiles,
                scratch);
   launch_early(k_na_sort, dim3(ntiles), dim3(kRadixThreads), 0, s, true, keys_in, keys_out, perm_out, n, ntiles,
-               scratch);
+               scratch, spin_limit, withheld_tile);
+  launch_early(k_na_again, dim3(1), dim3(kRadixThreads), 0, s, true, keys_in, keys_out, perm_out, n, ntiles, scratch);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     clsph_set_last_error(std::string("sort_keys_noalloc: launch: ") + cudaGetErrorString(e));
     return CLSPH_ERR_CUDA;
   }
   return CLSPH_OK;
+}
+
+extern "C" int clsph_gpu_sort_keys_noalloc(const uint32_t* keys_in, uint32_t* keys_out,
+                                           uint32_t* perm_out, uint32_t n, void* stream) {
+  return clsph_gpu_sort_keys_noalloc_limited(keys_in, keys_out, perm_out, n, stream, kRadixLookbackSpins, kNoTile);
 }

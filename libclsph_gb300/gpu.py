@@ -58,6 +58,7 @@ SIGNATURES = [
      [_vp, ctypes.c_int, ctypes.c_char_p, ctypes.c_int, _vp, _vp, ctypes.POINTER(ctypes.c_int)]),
     ("clsph_gpu_counters", ctypes.c_int, [_vp, _vp]),
     ("clsph_gpu_sort_keys_noalloc", ctypes.c_int, [_vp, _vp, _vp, _u32, _vp]),
+    ("clsph_gpu_sort_keys_noalloc_limited", ctypes.c_int, [_vp, _vp, _vp, _u32, _vp, _u32, _u32]),
     ("clsph_gpu_autotune", ctypes.c_int, [_vp, _u32, ctypes.c_char_p, ctypes.c_int]),
     ("clsph_gpu_set_launch_shape", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _u32]),
     ("clsph_gpu_set_neighbour_search", ctypes.c_int, [_vp, ctypes.c_int]),
