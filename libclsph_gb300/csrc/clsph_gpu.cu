@@ -126,7 +126,7 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
   // early 0.0938 / 0.0813 / 0.0787 ms of host time; a frame of 1,048,576
   // 6.240 / 6.226 / 7.859.
   const bool early = h->search == CLSPH_SEARCH_PARTICLE_WARPS;
-  h->launch_next(true, K_GRID_SETUP, k_grid_setup, dim3(1), dim3(256), h->bbox, h->grids,
+  h->launch_first(K_GRID_SETUP, k_grid_setup, dim3(1), dim3(256), h->bbox, h->grids,
             (const float*)h->scene_h, h->nscenes, h->status, h->digit_total, h->step_counters,
             h->ctl);
   // k_keys also clears the cell index (slots is a power of two >= 1024) and the sort's look-back words
@@ -739,7 +739,7 @@ int clsph_gpu_upload(clsph_gpu* h, const clsph_particle* particles) {
                              cudaMemcpyHostToDevice, h->stream));
     src = h->aos_stage;
   }
-  h->launch_next(true, K_MISC, k_bbox_reset, dim3(grid_blocks(6 * h->nscenes, 64)), dim3(kBlock), h->bbox,
+  h->launch_first(K_MISC, k_bbox_reset, dim3(grid_blocks(6 * h->nscenes, 64)), dim3(kBlock), h->bbox,
             h->nscenes);
   h->launch_next(true, K_UNPACK, k_unpack_aos, aos_grid(h), dim3(kBlock), src, h->n, h->st[0],
             (const uint16_t*)h->scene_of, h->bbox, h->status);
@@ -753,7 +753,7 @@ int clsph_gpu_download(clsph_gpu* h, clsph_particle* particles) {
   if (!h || !particles) return fail(CLSPH_ERR_ARGUMENT, "download: bad argument");
   if (!h->uploaded || h->partial) return fail(CLSPH_ERR_STATE, "download: no complete state");
   float4* dst = static_cast<float4*>(mapped_host_records(particles));
-  h->launch_next(true, K_PACK, k_pack_aos, aos_grid(h), dim3(kBlock), dst ? dst : h->aos_stage, h->n, h->st[0],
+  h->launch_first(K_PACK, k_pack_aos, aos_grid(h), dim3(kBlock), dst ? dst : h->aos_stage, h->n, h->st[0],
             (const float4*)h->aux, (const uint32_t*)h->keys, (const uint32_t*)h->ctl,
             h->have_fields ? 1 : 0);
   if (!dst)

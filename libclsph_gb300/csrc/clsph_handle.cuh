@@ -215,6 +215,15 @@ struct clsph_gpu {
     timed(cls, [&] { launch_early(k, g, b, 0, stream, early, args...); });
   }
 
+  // The first kernel after work that may not be the handle's own: on a caller's
+  // stream it waits, as a plain launch does, for everything queued before. (The
+  // wait of a kernel placed early covers the kernel before it only, and a
+  // caller's kernel may end without having waited for its own predecessors.)
+  template <typename Kernel, typename... Args>
+  void launch_first(int cls, Kernel k, dim3 g, dim3 b, Args... args) {
+    launch_next(stream == own_stream, cls, k, g, b, args...);
+  }
+
   template <typename Kernel, typename... Args>
   void launch_smem(int cls, Kernel k, dim3 g, dim3 b, size_t smem, Args... args) {
     timed(cls, [&] { k<<<g, b, smem, stream>>>(args...); });

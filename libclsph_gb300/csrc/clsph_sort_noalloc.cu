@@ -24,11 +24,11 @@
 //    before any stream capture.
 // It makes no cudaMalloc, cudaFree or other allocating call.
 //
-// Bound: the sort's own latencies (clsph_radix.cuh). Four launches, each with
-// its blocks placed while the one before still runs: 1,048,576 keys of 22 bits
-// 37 us, against 91 with a launch per pass and step. Without the last launch,
-// which is there for a wait that ran out, 35; without it and with a memset node
-// and plain launches 46 (39 with the memset alone).
+// Bound: the sort's own latencies (clsph_radix.cuh). Four launches, all but the
+// first with their blocks placed while the one before still runs: 1,048,576 keys of 22 bits
+// 39 us, against 91 with a launch per pass and step. With the first launch
+// placed early too 37, without the last one, which is there for a wait that ran
+// out, 35; without it, all launched in the plain way behind a memset node, 46.
 
 #include <cuda_runtime.h>
 
@@ -183,7 +183,9 @@ extern "C" int clsph_gpu_sort_keys_noalloc_limited(const uint32_t* keys_in, uint
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const uint32_t ntiles = (n + kRadixTile - 1) / kRadixTile;
   const uint32_t blocks = (n + kThreads - 1) / kThreads;
-  launch_early(k_na_clear, dim3(1), dim3(kThreads), 0, s, true, scratch);
+  // the first launch is a plain one: it waits for all earlier work of the caller's stream, also where the kernel just
+  // before was itself placed early and ends without having waited for its own predecessors
+  launch_early(k_na_clear, dim3(1), dim3(kThreads), 0, s, false, scratch);
   launch_early(k_na_count, dim3(blocks < 608u ? blocks : 608u), dim3(kThreads), 0, s, true, keys_in, n, ntiles,
                scratch);
   launch_early(k_na_sort, dim3(ntiles), dim3(kRadixThreads), 0, s, true, keys_in, keys_out, perm_out, n, ntiles,
