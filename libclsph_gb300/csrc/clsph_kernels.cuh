@@ -976,14 +976,22 @@ static __global__ void __launch_bounds__(kParticleWarps * 32)
 // ballot took 104 M (each list's far half is read and dropped, and a list
 // rarely fills its warps); planes cost one bit per particle and axis half.
 //
-// Rounding of the cull, in units of h. Candidates that matter lie within 1 of
-// a particle inside the own cell: |p'| <= sqrt(3), |q'| < 2.74, |q'|^2 < 7.5.
-// Rounding p' and q' to 11 bits moves 2 p'.q' by at most 2 (2.74 * 4.3e-4 +
-// 1.74 * 8.5e-4) < 5.4e-3; storing |q'|^2 and the three packed FMAs round
-// values below 8, at most 2^-9 each: 7.9e-3 in all. |p'|^2 - R^2 is rounded
-// down. So every candidate within h passes with R^2 = 1.015 > 1 + 1.33e-2;
-// the exact evaluation decides.
+// Rounding of the cull, in units of h, for a particle whose coordinates are at
+// most g = 1 + 1/64 (kCellGate; others, in cells whose centre is rounded far
+// from the origin, are not served) and a candidate within 1 of it:
+// |p'| < 1.76, |q'| < 2.76, |q'|^2 < 7.62.
+//  2 p' (below 4) is off by 2^-10 a component: 2^-10 sqrt(3) 2.76 = 4.7e-3 in
+//   the product; q' by 2^-11 a component below 2: 2 g 3 * 2^-11 = 3.0e-3, or
+//   2^-10 for one above 2 (then p' and q' lie close together in the other two,
+//   and the sums are 4.2e-3 and 4.0e-3): 8.2e-3 in all;
+//  |q'|^2 and the first FMA are below 8, 2^-9 each; the second below 4, 2^-10
+//   (if not, p' is near an axis and the product's share below 5.6e-3); the last,
+//   |p'|^2 - |p' - q'|^2, below 4, 2^-10: 5.9e-3.
+// 1.41e-2 in all (1.40e-2 is the largest of 10^7 draws; at 1.25 it would be
+// 1.76e-2), and |p'|^2 - R^2 is rounded down. So every candidate within h
+// passes with R^2 = 1.015; the exact evaluation decides.
 constexpr float kCellCullR2 = 1.015f;
+constexpr float kCellGate = 1.015625f;
 constexpr uint32_t kCellOffBits = kTagOffBits;
 
 // Per neighbour offset k (z, y, x order): the half-code bits a candidate of
@@ -1257,7 +1265,7 @@ __device__ __forceinline__ void density_cells_team(
       const uint32_t o = (up & 1u) | ((up >> 1) & 2u) | ((up >> 2) & 4u);
       uint32_t nc = cell.chunks[o];
       const bool served = valid && ((code ^ up) & 0x15u) == 0x15u &&
-                          fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) < 1.25f && nc <= 4u * kWords;
+                          fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= kCellGate && nc <= 4u * kWords;
       if (!served) nc = 0u;
       const uint32_t nw = (__reduce_max_sync(0xFFFFFFFFu, nc) + 3u) >> 2;
       const __half2 px = __float2half2_rn(2.f * x), py = __float2half2_rn(2.f * y), pz = __float2half2_rn(2.f * z);
