@@ -112,6 +112,16 @@ struct DevMesh {
   float reach;  // longest segment a cell list covers
 };
 
+// Loads of what a substep's own phases write (positions, cell index, neighbour
+// starts and records, ...): read-only loads where each phase is a kernel of its
+// own; plain ones (kLive) in the persistent kernel, which writes these arrays
+// in the launch that reads them.
+template <bool kLive, typename T>
+__device__ __forceinline__ T ld_step(const T* p) {
+  if constexpr (kLive) return *p;
+  else return __ldg(p);
+}
+
 // ------------------------------------------------------------ cell index
 __device__ __forceinline__ uint32_t cell_slot_insert(const CellIndex& ci, uint32_t key) {
   const uint32_t tag = key + 1u;
@@ -124,12 +134,13 @@ __device__ __forceinline__ uint32_t cell_slot_insert(const CellIndex& ci, uint32
   return 0xFFFFFFFFu;  // unreachable: at most n keys in >= 2n slots
 }
 
+template <bool kLive = false>
 __device__ __forceinline__ uint2 cell_lookup(const CellIndex& ci, uint32_t key) {
   const uint32_t tag = key + 1u;
   uint32_t slot = cell_hash(key) >> ci.shift;
   for (uint32_t probe = 0; probe <= ci.mask; ++probe) {
-    uint32_t k = __ldg(&ci.keys[slot]);
-    if (k == tag) return make_uint2(__ldg(&ci.start[slot]), __ldg(&ci.end[slot]));
+    uint32_t k = ld_step<kLive>(&ci.keys[slot]);
+    if (k == tag) return make_uint2(ld_step<kLive>(&ci.start[slot]), ld_step<kLive>(&ci.end[slot]));
     if (k == 0u) break;
     slot = (slot + 1u) & ci.mask;
   }
@@ -839,6 +850,7 @@ __device__ __forceinline__ bool near_cull(const float4& p, const float4& q, floa
   return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= r2;
 }
 
+template <bool kLive = false>
 __device__ __forceinline__ void density_particle_warp(
     uint32_t i, uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
     const KeySplit& split, const uint32_t* __restrict__ keys, const float4* __restrict__ pos, const CellIndex& ci,
@@ -867,7 +879,7 @@ __device__ __forceinline__ void density_particle_warp(
                    z = (uint32_t)cc[2] + lane / 9u - 1u;
     inw = x >= w.lo[0] && x <= w.hi[0] && y >= w.lo[1] && y <= w.hi[1] && z >= w.lo[2] && z <= w.hi[2];
     if (inw) {
-      const uint2 r = cell_lookup(ci, morton3(x, y, z) | sbits);
+      const uint2 r = cell_lookup<kLive>(ci, morton3(x, y, z) | sbits);
       cs = r.x;
       ce = r.y;
     }
@@ -885,7 +897,7 @@ __device__ __forceinline__ void density_particle_warp(
       bool hit = false;
       float term = 0.f;
       if (j < r.y) {
-        const float4 pj = __ldg(&pos[j]);
+        const float4 pj = ld_step<kLive>(&pos[j]);
         if ((__float_as_uint(pj.w) & need) == need && near_cull(pi, pj, cull_r2)) {
           const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
           const float rr = xnorm(d);
@@ -1054,6 +1066,7 @@ struct CellTeamSmem {
 constexpr uint32_t kNoLists = 0xFFFFFFFEu, kNoCell = 0xFFFFFFFFu;
 
 // The slots of word `w` of the planes in [s, e) that have all of `need`.
+template <bool kLive>
 __device__ __forceinline__ uint32_t facing_slots(const uint32_t* __restrict__ planes, uint32_t w, uint32_t s,
                                                  uint32_t e, uint32_t need) {
   const uint32_t* p = planes + (size_t)w * kHalfPlanes;
@@ -1061,7 +1074,7 @@ __device__ __forceinline__ uint32_t facing_slots(const uint32_t* __restrict__ pl
 #pragma unroll
   for (uint32_t b = 0; b < kHalfPlanes; b += 2) {  // an axis needs at most one of its two bits
     const uint32_t both = (need >> b) & 3u;
-    const uint32_t v = __ldg(&p[b + (both >> 1)]);  // (loaded in any case: the loads don't wait for one another)
+    const uint32_t v = ld_step<kLive>(&p[b + (both >> 1)]);  // (loaded in any case: the loads don't wait for one another)
     m &= both ? v : 0xFFFFFFFFu;
   }
   const uint32_t w0 = 32u * w;
@@ -1070,7 +1083,7 @@ __device__ __forceinline__ uint32_t facing_slots(const uint32_t* __restrict__ pl
   return m;
 }
 
-template <class Team>
+template <bool kLive = false, class Team>
 __device__ __forceinline__ void density_cells_team(
     uint32_t n, const DevGrid* __restrict__ grids, const uint32_t* __restrict__ ctl,
     const uint16_t* __restrict__ scene_of, const uint32_t* __restrict__ keys_base, const float4* __restrict__ pos,
@@ -1092,8 +1105,8 @@ __device__ __forceinline__ void density_cells_team(
   const KeySplit split{ctl[kCtlShift]};
   const bool whole_keys = split.shift + ctl[kCtlSceneBits] <= 32u;  // (if not, flagged, keys lose upper scene bits)
   auto by_warp = [&](uint32_t i) {
-    density_particle_warp(i, n, grids, scene_of, split, keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n, pos, ci,
-                          consts, aux_out, nlist, ncount, nlist_cap, vel, frec, nb_start);
+    density_particle_warp<kLive>(i, n, grids, scene_of, split, keys_base + (size_t)sorted_sel(ctl[kCtlMaxKey]) * n,
+                                 pos, ci, consts, aux_out, nlist, ncount, nlist_cap, vel, frec, nb_start);
   };
   // the last warp, which has the fewest particles, looks the next cell up; the first two cells have fixed
   // numbers, the others come from the work counter, and both are loaded a cell ahead
@@ -1103,7 +1116,7 @@ __device__ __forceinline__ void density_cells_team(
   bool have = false;
   auto load_entry = [&]() {
     have = ticket < ncells;
-    if (have) entry = __ldg(&cell_list[ticket]);
+    if (have) entry = ld_step<kLive>(&cell_list[ticket]);
   };
   if (fetcher) {
     load_entry();
@@ -1120,7 +1133,7 @@ __device__ __forceinline__ void density_cells_team(
       if (lane < 27u) {
         const uint32_t x = compact_bits3(key) + lane % 3u - 1u, y = compact_bits3(key >> 1) + (lane / 3u) % 3u - 1u,
                        z = compact_bits3(key >> 2) + lane / 9u - 1u;
-        const uint2 r = cell_lookup(ci, morton3(x, y, z) | (own.y ^ key));
+        const uint2 r = cell_lookup<kLive>(ci, morton3(x, y, z) | (own.y ^ key));
         s = lane == 13u ? own.x : r.x;  // (a flagged sort stall can leave the index with another start)
         e = r.y;
         nb_start[(size_t)own.x * 27u + lane] = s;
@@ -1141,16 +1154,17 @@ __device__ __forceinline__ void density_cells_team(
 #pragma unroll
         for (uint32_t w = 0; w < 3u; ++w) {
           const bool on = w < words;
-          m[w] = facing_slots(planes, on ? w0 + w : 0u, on ? s : 0u, on ? e : 1u, need) & (on ? 0xFFFFFFFFu : 0u);
+          m[w] = facing_slots<kLive>(planes, on ? w0 + w : 0u, on ? s : 0u, on ? e : 1u, need) & (on ? 0xFFFFFFFFu : 0u);
         }
         if (count <= 32u) {  // only the neighbour cells in its particles' windows
           uint32_t any = 0;
           if (lane < kHalfPlanes)
-            for (uint32_t w = own.x >> 5; w <= (own_e - 1u) >> 5; ++w) any |= facing_slots(planes, w, own.x, own_e, 1u << lane);
+            for (uint32_t w = own.x >> 5; w <= (own_e - 1u) >> 5; ++w)
+              any |= facing_slots<kLive>(planes, w, own.x, own_e, 1u << lane);
           if (!((window_cells(__ballot_sync(0xFFFFFFFFu, any != 0u)) >> lane) & 1u)) m[0] = m[1] = m[2] = 0u;
         }
         uint32_t size = lane == 13u ? count : __popc(m[0]) + __popc(m[1]) + __popc(m[2]);
-        for (uint32_t w = 3; w < words; ++w) size += __popc(facing_slots(planes, w0 + w, s, e, need));
+        for (uint32_t w = 3; w < words; ++w) size += __popc(facing_slots<kLive>(planes, w0 + w, s, e, need));
         uint32_t end = size;
 #pragma unroll
         for (uint32_t d = 1; d < 32u; d <<= 1) {
@@ -1170,7 +1184,7 @@ __device__ __forceinline__ void density_cells_team(
               m[0] = m[1];
               m[1] = m[2];
               ++w;
-              m[2] = w < words ? facing_slots(planes, w0 + w, s, e, need) : 0u;
+              m[2] = w < words ? facing_slots<kLive>(planes, w0 + w, s, e, need) : 0u;
               tag += 32u;
             }
             sm.pend[at++] = (uint16_t)(tag + __ffs(m[0]) - 1u);
@@ -1232,7 +1246,7 @@ __device__ __forceinline__ void density_cells_team(
       for (uint32_t u = 0; u < kAhead; ++u) {
         const uint32_t e = min(e0 + 32u * kWarps * u, candidates - 1u);
         tag[u] = sm.pend[e];
-        q[u] = __ldg(&pos[cell.slot_of[tag[u] >> kCellOffBits] + tag[u]]);
+        q[u] = ld_step<kLive>(&pos[cell.slot_of[tag[u] >> kCellOffBits] + tag[u]]);
       }
 #pragma unroll
       for (uint32_t u = 0; u < kAhead; ++u) {
@@ -1307,7 +1321,7 @@ __device__ __forceinline__ void density_cells_team(
         const uint32_t b = 31u - __clz(m);
         m ^= 1u << b;
         tag = reinterpret_cast<const uint16_t*>(&sm.chunk[(ids >> (b & 24u)) & 255u][4])[b & 7u];
-        return __ldg(&pos[cell.slot_of[tag >> kCellOffBits] + tag]);
+        return ld_step<kLive>(&pos[cell.slot_of[tag >> kCellOffBits] + tag]);
       };
       uint32_t tag = 0;
       float4 pj = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1370,6 +1384,7 @@ struct NoForceHook {
 // added one after another in lane order, which is the reference's sequence.
 // (One lane alone walks its 500 to 1,000 candidates in about 150 us, which a
 // single such particle adds to the kernel; the warp takes a few us.)
+template <bool kLive = false>
 __device__ __forceinline__ void forces_particle_warp(uint32_t i, uint32_t n, const DevGrid* grids,
                                                      const uint16_t* scene_of, const uint32_t* ctl,
                                                      const uint32_t* keys_base, const State& st, const float4* aux,
@@ -1386,7 +1401,7 @@ __device__ __forceinline__ void forces_particle_warp(uint32_t i, uint32_t n, con
   for (uint32_t z = w.lo[2]; z <= w.hi[2]; ++z)
     for (uint32_t y = w.lo[1]; y <= w.hi[1]; ++y)
       for (uint32_t x = w.lo[0]; x <= w.hi[0]; ++x) {
-        const uint2 r = cell_lookup(ci, morton3(x, y, z) | split.scene_bits(sc));
+        const uint2 r = cell_lookup<kLive>(ci, morton3(x, y, z) | split.scene_bits(sc));
         for (uint32_t base = r.x; base < r.y; base += 32u) {
           const uint32_t j = base + lane;
           bool hit = false;
@@ -1454,7 +1469,7 @@ __device__ __forceinline__ void forces_particle_alone(uint32_t i, uint32_t n, co
 // average) 0.186 -> 0.155 ms, with the learned step's features 0.361 -> 0.256
 // (at most 102 registers: the features' 22 sums; unbounded, the compiler took
 // 113 and 0.310 ms).
-template <class Hook>
+template <bool kLive = false, class Hook>
 __device__ __forceinline__ void forces_particle(
     bool valid, uint32_t i, uint32_t n, const DevGrid* __restrict__ grids, const uint16_t* __restrict__ scene_of,
     const uint32_t* __restrict__ ctl, const uint32_t* __restrict__ keys_base, const State& st,
@@ -1482,7 +1497,7 @@ __device__ __forceinline__ void forces_particle(
     // its offset there; the own cell's nb_start row holds their first slots
     const uint32_t* nbs = nb_start + (size_t)__float_as_uint(ai.z) * 27u;
     auto slot = [&](uint32_t tag) {
-      return __ldg(&nbs[tag >> kTagOffBits]) + (tag & ((1u << kTagOffBits) - 1u));
+      return ld_step<kLive>(&nbs[tag >> kTagOffBits]) + (tag & ((1u << kTagOffBits) - 1u));
     };
     // software pipeline: while a pair is evaluated, the tag three pairs
     // ahead is loaded, the tag two ahead is resolved to its slot and the
@@ -1491,11 +1506,11 @@ __device__ __forceinline__ void forces_particle(
       uint32_t tnn = cnt > 2 ? t2 : cnt > 1 ? t1 : t0;
       uint32_t j = slot(t0);
       uint32_t jn = slot(cnt > 1 ? t1 : t0);
-      float4 pj = __ldg(&frec[j]), vj = __ldg(&frec[(size_t)n + j]);
+      float4 pj = ld_step<kLive>(&frec[j]), vj = ld_step<kLive>(&frec[(size_t)n + j]);
       for (uint32_t k = 0; k < cnt; ++k) {
         const uint32_t t3 = k + 3 < cnt ? tag_at(k + 3) : tnn;
         const uint32_t jnn = slot(tnn);
-        const float4 pn = __ldg(&frec[jn]), vn = __ldg(&frec[(size_t)n + jn]);
+        const float4 pn = ld_step<kLive>(&frec[jn]), vn = ld_step<kLive>(&frec[(size_t)n + jn]);
         const V3 d = {XSUB(pi.x, pj.x), XSUB(pi.y, pj.y), XSUB(pi.z, pj.z)};
         force_pair<true>(f, j == i, d, near_norm(d), vi, vj, pj.w, vj.w, own, hh, lap_b, c);
         // the same differences the terms use (the compiler shares them); dead
@@ -1515,8 +1530,8 @@ __device__ __forceinline__ void forces_particle(
   }
   if constexpr (!Hook::kPairs) {
     for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, valid && !listed); rest; rest &= rest - 1u)
-      forces_particle_warp(__shfl_sync(0xFFFFFFFFu, i, __ffs(rest) - 1), n, grids, scene_of, ctl, keys_base, st, aux,
-                           ci, consts, acc_out, frec);
+      forces_particle_warp<kLive>(__shfl_sync(0xFFFFFFFFu, i, __ffs(rest) - 1), n, grids, scene_of, ctl, keys_base, st,
+                                  aux, ci, consts, acc_out, frec);
   } else if (valid && !listed) {
     forces_particle_alone(i, n, grids, scene_of, ctl, keys_base, st, aux, ci, consts, acc_out, hook, frec);
   }

@@ -133,15 +133,15 @@ static __global__ void __launch_bounds__(kPersistThreads, 3)
       gather_block(vb, n, a.grids, a.scene_of, a.ctl, a.keys, a.vals, a.st[0], a.st[1], a.ids[src_ids],
                    a.ids[src_ids ^ 1u], a.ci, a.cell_list, a.step_counters + kCntCells, a.planes, sm.gather);
     if (!grid_barrier(a, ok_s)) return;
-    density_cells_team(n, a.grids, a.ctl, a.scene_of, a.keys, a.st[1].pos, a.planes, a.ci, a.consts, a.aux, a.nlist,
-                       a.ncount, a.nlist_cap, a.st[1].vel, a.frec, a.cell_list, a.step_counters, a.nb_start,
-                       sm.dens[threadIdx.x >> 6], (threadIdx.x >> 5) & 1u,
-                       blockIdx.x * (kPersistThreads / 64u) + (threadIdx.x >> 6), gridDim.x * (kPersistThreads / 64u),
-                       1u + (threadIdx.x >> 6));
+    density_cells_team<true>(n, a.grids, a.ctl, a.scene_of, a.keys, a.st[1].pos, a.planes, a.ci, a.consts, a.aux,
+                             a.nlist, a.ncount, a.nlist_cap, a.st[1].vel, a.frec, a.cell_list, a.step_counters,
+                             a.nb_start, sm.dens[threadIdx.x >> 6], (threadIdx.x >> 5) & 1u,
+                             blockIdx.x * (kPersistThreads / 64u) + (threadIdx.x >> 6),
+                             gridDim.x * (kPersistThreads / 64u), 1u + (threadIdx.x >> 6));
     if (!grid_barrier(a, ok_s)) return;
     for (uint32_t i = gtid; (i & ~31u) < n; i += gstride)
-      forces_particle(i < n, i, n, a.grids, a.scene_of, a.ctl, a.keys, a.st[1], a.aux, a.ci, a.consts, a.nlist, a.ncount,
-                      a.nlist_cap, a.acc, NoForceHook{}, a.frec, a.nb_start);
+      forces_particle<true>(i < n, i, n, a.grids, a.scene_of, a.ctl, a.keys, a.st[1], a.aux, a.ci, a.consts, a.nlist,
+                            a.ncount, a.nlist_cap, a.acc, NoForceHook{}, a.frec, a.nb_start);
     if (!grid_barrier(a, ok_s)) return;
     advect_blocks<false>(blockIdx.x, gridDim.x, n, a.st[1], a.acc, a.st[0], a.meshes, a.consts, a.scene_of,
                          a.max_iters, a.bbox, a.status, a.capped, nullptr, 1.f, 1.f, nullptr, nullptr, sm.bbox);
