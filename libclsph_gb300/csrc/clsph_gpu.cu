@@ -82,6 +82,15 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
   return c;
 }
 
+// The form of the cell search for the scenes' fluids, and the team that a
+// handle takes whose launch shapes nobody has set.
+void choose_lists(clsph_gpu* h) {
+  h->packed_cells = false;
+  for (const Consts& c : h->consts_host)
+    if (!(8.f * c.h * c.h * c.h * c.rho0 <= 50.f * c.mass)) h->packed_cells = true;
+  if (!h->shapes_set) h->density_block = h->packed_cells || h->n <= 64000u ? 128 : 64;
+}
+
 // Launch shapes of a new handle (clsph_gpu_set_neighbour_search,
 // clsph_gpu_set_launch_shape and clsph_gpu_autotune replace them). Measured
 // (density kernel, us; one warp per particle / teams of 4 / of 2 warps):
@@ -96,10 +105,8 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
 // the larger lists: shared memory for 92 chunks lets 16 teams of two share an
 // SM, for 128 chunks 12 (1,048,576 particles of water: 0.309 against 0.346 ms).
 void choose_shapes(clsph_gpu* h) {
-  for (const Consts& c : h->consts_host)
-    if (!(8.f * c.h * c.h * c.h * c.rho0 <= 50.f * c.mass)) h->packed_cells = true;
+  choose_lists(h);
   h->search = h->n <= 14000u ? CLSPH_SEARCH_PARTICLE_WARPS : CLSPH_SEARCH_CELL_WARPS;
-  h->density_block = h->packed_cells || h->n <= 64000u ? 128 : 64;
   // advection blocks per SM: blocks of 1,000 to 2,000 consecutive particles even out their collisions
   // (4,194,304 particles on a heightfield: 8 / 16 / 32 / 64 blocks 0.329 / 0.295 / 0.289 / 0.311 ms; 1,048,576
   // on a floor: 8 / 16 0.038 / 0.041)
@@ -848,6 +855,9 @@ int clsph_gpu_set_scene_parameters(clsph_gpu* h, uint32_t scene, const clsph_par
   h->params[scene] = p;
   h->terms[scene] = *terms;
   h->consts_host[scene] = derive_consts(p, *terms, count);
+  const bool packed = h->packed_cells;
+  choose_lists(h);
+  if (h->packed_cells != packed) h->drop_graph();  // the captured launches have the other lists
   const float hs = p.h;
   CUDA_TRY(cudaMemcpyAsync(h->scene_h + scene, &hs, sizeof(float), cudaMemcpyHostToDevice, h->stream));
   return sync_scene_tables(h);
@@ -1038,6 +1048,7 @@ int clsph_gpu_autotune(clsph_gpu* h, uint32_t substeps, char* report, int report
   h->density_block = best_d;
   h->forces_block = best_f;
   h->search = best_s;
+  h->shapes_set = true;
   const uint32_t advect_opts[3] = {4, 8, 16};
   uint32_t best_a = h->advect_blocks_per_sm;
   double ta = 1e30;
@@ -1115,6 +1126,7 @@ int clsph_gpu_set_launch_shape(clsph_gpu* h, int density_block, int forces_block
   h->density_block = density_block;
   h->forces_block = forces_block;
   h->advect_blocks_per_sm = advect_blocks_per_sm;
+  h->shapes_set = true;
   h->drop_graph();
   return CLSPH_OK;
 }
