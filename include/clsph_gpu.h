@@ -231,7 +231,8 @@ int clsph_gpu_set_launch_shape(clsph_gpu* h, int density_block, int forces_block
  * above. The density block size of clsph_gpu_set_launch_shape sets WINDOW's
  * block (64 or 128 threads; 256 runs as 128) and the team of CELL_WARPS (64 /
  * 128 / 256 threads = 2 / 4 / 8 warps); clsph_gpu_autotune tries every
- * combination. */
+ * combination. A handle with a scene whose h is outside 2^-20 .. 2^20 runs one
+ * of the other two in place of CELL_WARPS (and of the persistent form below). */
 enum {
   CLSPH_SEARCH_WINDOW = 0,
   CLSPH_SEARCH_CELL_WARPS = 1,

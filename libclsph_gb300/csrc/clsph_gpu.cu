@@ -83,11 +83,17 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
 }
 
 // The form of the cell search for the scenes' fluids, and the team that a
-// handle takes whose launch shapes nobody has set.
+// handle takes whose launch shapes nobody has set. The teams' square root wants
+// every h within 2^-20 .. 2^20; a handle with another runs one of the searches
+// that evaluate the general one (the same results): 32,768 particles, a warp
+// per particle / a thread per particle 57 / 90 us, 131,072 207 / 115, 1,048,576
+// 1632 / 665.
 void choose_lists(clsph_gpu* h) {
-  h->packed_cells = false;
-  for (const Consts& c : h->consts_host)
+  h->packed_cells = h->general_h = false;
+  for (const Consts& c : h->consts_host) {
     if (!(8.f * c.h * c.h * c.h * c.rho0 <= 50.f * c.mass)) h->packed_cells = true;
+    if (!c.plain_h) h->general_h = true;
+  }
   if (!h->shapes_set) h->density_block = h->packed_cells || h->n <= 64000u ? 128 : 64;
 }
 
@@ -132,7 +138,9 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
   // A callback substep of 4,096 particles: none / all but these two / all placed
   // early 0.0938 / 0.0813 / 0.0787 ms of host time; a frame of 1,048,576
   // 6.240 / 6.226 / 7.859.
-  const bool early = h->search == CLSPH_SEARCH_PARTICLE_WARPS;
+  const int search = h->search != CLSPH_SEARCH_CELL_WARPS || !h->general_h ? h->search
+                     : n <= 64000u ? CLSPH_SEARCH_PARTICLE_WARPS : CLSPH_SEARCH_WINDOW;
+  const bool early = search == CLSPH_SEARCH_PARTICLE_WARPS;
   h->launch_first(K_GRID_SETUP, k_grid_setup, dim3(1), dim3(256), h->bbox, h->grids,
             (const float*)h->scene_h, h->nscenes, h->status, h->digit_total, h->step_counters,
             h->ctl);
@@ -177,12 +185,12 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
                 (const float4*)h->st[1].vel, h->frec, (const uint2*)h->cell_list,
                 h->step_counters, h->nb_start);
     };
-    if (h->search == CLSPH_SEARCH_CELL_WARPS) {
+    if (search == CLSPH_SEARCH_CELL_WARPS) {
       if (h->density_block == 256) cells(k_density_cells<CellTeamSmem<8, 128, 14>, 3>, 3, 8);
       else if (h->density_block == 128) cells(k_density_cells<CellTeamSmem<4, 128, 14>, 7>, 2, 4);
       else if (h->packed_cells) cells(k_density_cells<CellTeamSmem<2, 128, 14>, 12>, 1, 2);
       else cells(k_density_cells<CellTeamSmem<2, 92, 11>, 16>, 0, 2);
-    } else if (h->search == CLSPH_SEARCH_PARTICLE_WARPS) {
+    } else if (search == CLSPH_SEARCH_PARTICLE_WARPS) {
       h->launch_next(early, K_DENSITY, k_density_pwarp, dim3((n + kParticleWarps - 1) / kParticleWarps),
                 dim3(kParticleWarps * 32), n, (const DevGrid*)h->grids, (const uint16_t*)h->scene_of,
                 cctl, (const uint32_t*)h->keys, (const float4*)h->st[1].pos, h->ci,
@@ -774,7 +782,7 @@ int clsph_gpu_step(clsph_gpu* h, uint32_t substeps) {
   if (!h) return fail(CLSPH_ERR_ARGUMENT, "step: null handle");
   if (!h->uploaded || h->partial) return fail(CLSPH_ERR_STATE, "step: upload particles first");
   uint32_t done = 0;
-  if (h->persistent && !h->profiling) {
+  if (h->persistent && !h->profiling && !h->general_h) {
     int rc = launch_persistent(h, substeps);
     if (rc) return rc;
     h->substeps += substeps;
@@ -855,9 +863,9 @@ int clsph_gpu_set_scene_parameters(clsph_gpu* h, uint32_t scene, const clsph_par
   h->params[scene] = p;
   h->terms[scene] = *terms;
   h->consts_host[scene] = derive_consts(p, *terms, count);
-  const bool packed = h->packed_cells;
+  const bool packed = h->packed_cells, general = h->general_h;
   choose_lists(h);
-  if (h->packed_cells != packed) h->drop_graph();  // the captured launches have the other lists
+  if (h->packed_cells != packed || h->general_h != general) h->drop_graph();  // the captured launches have the other form
   const float hs = p.h;
   CUDA_TRY(cudaMemcpyAsync(h->scene_h + scene, &hs, sizeof(float), cudaMemcpyHostToDevice, h->stream));
   return sync_scene_tables(h);

@@ -150,6 +150,7 @@ struct clsph_gpu {
   int density_block = 128;
   int search = CLSPH_SEARCH_CELL_WARPS;  // neighbour search of the density kernel
   bool shapes_set = false;    // by clsph_gpu_set_launch_shape or clsph_gpu_autotune
+  bool general_h = false;     // some scene's h is outside the cell search's range
   bool packed_cells = false;  // some scene's fluid at rest has more than 50 particles in a 2h cell
   uint32_t density_resident[4] = {};  // resident blocks of each form of the cell search (0: not yet asked)
   int forces_block = 128;

@@ -973,8 +973,9 @@ static __global__ void __launch_bounds__(kParticleWarps * 32)
 // serve are done by a whole warp each (density_particle_warp): those on a
 // mid-plane of the cell, so in two octants; cells of up to kSparseCell
 // particles, for which the lists cost more than they save; lists longer than
-// the team's shared memory; neighbours of a cell of 2048 or more particles,
-// which tags can't address; and scenes whose h is outside near_norm's range.
+// the team's shared memory; and neighbours of a cell of 2048 or more particles,
+// which tags can't address. Every scene's h lies in near_norm's range (handles
+// with another take a search of their own).
 //
 // Bound: instruction issue, half of it the exact evaluation. 1,048,576
 // particles spread over a floor (29,552 cells, a quarter of them of one or
@@ -1146,7 +1147,7 @@ __device__ __forceinline__ void density_cells_team(
       const uint32_t count = own_e > own.x ? own_e - own.x : 0u;
       uint32_t candidates = kNoLists;
       const uint32_t sc = whole_keys ? (split.shift >= 32u ? 0u : own.y >> split.shift) : scene_of[own.x];
-      if (!__any_sync(0xFFFFFFFFu, e - s >= (1u << kCellOffBits)) && count > kSparseCell && consts[sc].plain_h) {
+      if (!__any_sync(0xFFFFFFFFu, e - s >= (1u << kCellOffBits)) && count > kSparseCell) {
         // the candidates of list k as bits, in up to three words of the planes (more are counted and read again)
         const uint32_t need = kOffsetMasks.m[min(lane, 26u)];
         const uint32_t w0 = s >> 5, words = e > s && lane != 13u ? ((e - 1u) >> 5) - w0 + 1u : 0u;
