@@ -213,9 +213,10 @@ int clsph_gpu_kernel_times(clsph_gpu* h, int max_classes, char* names, int name_
 int clsph_gpu_autotune(clsph_gpu* h, uint32_t substeps, char* report, int report_len);
 
 /* Sets the launch shapes directly (e.g. from a cached autotune result):
- * blocks of 64, 128 or 256 threads; 1..64 advection blocks per SM. (Scenes of
+ * blocks of 64, 128 or 256 threads; 1..64 advection blocks per SM. (Handles of
  * up to 40,000 particles run the forces with several lanes per particle in
- * blocks of their own size.) */
+ * blocks of their own size; forces_block is then the learned step's, whose
+ * feature kernel has one lane per particle.) */
 int clsph_gpu_set_launch_shape(clsph_gpu* h, int density_block, int forces_block,
                                uint32_t advect_blocks_per_sm);
 

@@ -218,8 +218,8 @@ int clsph_host::enqueue_substep(clsph_gpu* h, int until) {
                 (const float4*)h->aux, h->ci, (const Consts*)h->consts, (const uint16_t*)h->nlist,
                 (const uint32_t*)h->ncount, h->nlist_cap, h->acc, (const float4*)h->frec, (const uint32_t*)h->nb_start);
     };
-    if (n <= kWide8) wide(k_forces_wide<8>, 8);
-    else if (n <= kWide4) wide(k_forces_wide<4>, 4);
+    if (n <= kWide8 && !h->one_lane_forces) wide(k_forces_wide<8>, 8);
+    else if (n <= kWide4 && !h->one_lane_forces) wide(k_forces_wide<4>, 4);
     else if (b == 64) args(k_forces<64>);
     else if (b == 256) args(k_forces<256>);
     else args(k_forces<128>);
@@ -1049,7 +1049,9 @@ int clsph_gpu_autotune(clsph_gpu* h, uint32_t substeps, char* report, int report
              std::to_string(d) + " ms\n";
       if (d < td) { td = d; best_d = b; best_s = sm; }
     }
+    h->one_lane_forces = true;  // the form whose block is chosen here, also where only the learned step runs it
     double f = trial(K_FORCES);
+    h->one_lane_forces = false;
     out += "forces block " + std::to_string(b) + ": " + std::to_string(f) + " ms\n";
     if (f < tf) { tf = f; best_f = b; }
   }

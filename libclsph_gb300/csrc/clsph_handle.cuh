@@ -153,7 +153,8 @@ struct clsph_gpu {
   bool general_h = false;     // some scene's h is outside the cell search's range
   bool packed_cells = false;  // some scene's fluid at rest has more than 50 particles in a 2h cell
   uint32_t density_resident[4] = {};  // resident blocks of each form of the cell search (0: not yet asked)
-  int forces_block = 128;
+  int forces_block = 128;        // of the forms with one lane per particle
+  bool one_lane_forces = false;  // clsph_gpu_autotune times that form whatever the handle's size
   uint32_t advect_blocks_per_sm = 8;
 
   // the substep loop as one persistent cooperative launch (clsph_persistent.cuh)
