@@ -74,9 +74,9 @@ Consts derive_consts(const clsph_parameters& p, const clsph_kernel_terms& t, uin
   c.visc = t.viscosity;
   // smoothing.cl:24: -45 / (float)(M_PI * pown(h, 6)) with M_PI in double
   c.spiky_zero = -45.f / (float)(M_PI * (double)pown_f(p.h, 6));
-  // conservative h^2 of the FMA culls: 5e-4 above h^2, five times the largest
-  // rounding of the cell-relative cull (k_density_cells) and far above that
-  // of the direct differences; the exact test decides
+  // conservative h^2 of the FMA culls on direct differences: 5e-4 above h^2, far
+  // above their rounding; the exact test decides (the cell search has a cull of
+  // its own, kCellCullR2)
   c.cull_r2 = p.h * p.h * 1.0005f;
   c.plain_h = p.h >= 0x1p-20f && p.h <= 0x1p20f;
   return c;
@@ -115,7 +115,8 @@ void choose_shapes(clsph_gpu* h) {
   h->search = h->n <= 14000u ? CLSPH_SEARCH_PARTICLE_WARPS : CLSPH_SEARCH_CELL_WARPS;
   // advection blocks per SM: blocks of 1,000 to 2,000 consecutive particles even out their collisions
   // (4,194,304 particles on a heightfield: 8 / 16 / 32 / 64 blocks 0.329 / 0.295 / 0.289 / 0.311 ms; 1,048,576
-  // on a floor: 8 / 16 0.038 / 0.041)
+  // on a floor: 8 / 16 0.038 / 0.041; on the dam break, where few collide, 4 / 8 / 16 0.027 / 0.031 / 0.035, which
+  // the autotuner finds)
   h->advect_blocks_per_sm = h->n > 2000000u ? 16u : 8u;
 }
 

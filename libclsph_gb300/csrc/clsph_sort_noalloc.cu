@@ -25,10 +25,11 @@
 // It makes no cudaMalloc, cudaFree or other allocating call.
 //
 // Bound: the sort's own latencies (clsph_radix.cuh). Four launches, all but the
-// first with their blocks placed while the one before still runs: 1,048,576 keys of 22 bits
-// 39 us, against 91 with a launch per pass and step. With the first launch
-// placed early too 37, without the last one, which is there for a wait that ran
-// out, 35; without it, all launched in the plain way behind a memset node, 46.
+// first with their blocks placed while the one before still runs: 1,048,576
+// keys of 22 bits 39 us, against 91 with a launch per pass and step. With the
+// first launch placed early too 37; without the last one, which is there for a
+// wait that ran out, 35; without it, all launched in the plain way behind a
+// memset node, 46.
 
 #include <cuda_runtime.h>
 
