@@ -1076,7 +1076,7 @@ int clsph_gpu_autotune(clsph_gpu* h, uint32_t substeps, char* report, int report
   int coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
   bool use_persistent = false;
-  if (coop) {
+  if (coop && !h->general_h) {  // (such a handle runs launched substeps in any case)
     const uint32_t even = std::max<uint32_t>(2u, substeps & ~1u);
     const bool graph0 = h->use_graph;
     cudaEvent_t e0 = take_event_of(h), e1 = take_event_of(h);

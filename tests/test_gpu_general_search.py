@@ -51,3 +51,12 @@ def test_radius_leaves_and_enters_the_range(gpu_lib):
             g.upload((a, b)[k])
             g.step(2)
             assert np.array_equal(g.download().view(np.uint8), want[k].view(np.uint8))
+
+
+def test_autotune_offers_no_persistent_form(gpu_lib):
+    """Out of range the persistent form is not run: a report would compare the launched one with itself."""
+    p, t, pos, vel, mesh, _ = _block(12, 0.99 * 2.0 ** -20 / float(W.water_settings(12 ** 3).params["h"]))
+    with GpuSolver(p, t, len(pos), mesh) as g:
+        g.upload(W.particles_from_arrays(pos, vel, vel))
+        report = g.autotune(2)
+    assert "whole substep" not in report and "launched substeps" in report
