@@ -230,7 +230,7 @@ __device__ __forceinline__ void grid_setup_block(uint32_t* __restrict__ bbox_all
   g.half_margin = (float)(gmax + 2) * 0x1p-20f;
   for (int i = 0; i < 4; ++i) g.pad_[i] = 0u;
   *grid = g;
-  if (overflow) {  // (flagged) cells holds the wrapped sizes, and coordinates wrap at ten bits: take all the bits there are
+  if (overflow) {  // cells holds the wrapped sizes, while coordinates wrap at ten bits: take all the bits there are
     atomicOr(status, kFlagGridOverflow);
     atomicMax(&shift_s, min(30u, 32u - ctl[kCtlSceneBits]));
   }

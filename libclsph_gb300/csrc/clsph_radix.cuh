@@ -18,10 +18,10 @@
 // wait is bounded all the same (spin_limit, by default kRadixLookbackSpins),
 // and one that runs out raises kFlagSortStall, which clsph_gpu_sync reports as
 // an error (the stand-alone sort, which has no later call to report it, sorts
-// again in one block). After a stall the offsets of the tiles behind it are wrong, but
-// every store stays in bounds (destinations >= n are skipped, and the slots a
-// pass leaves unwritten keep earlier in-range values), so the context stays
-// usable.
+// again in one block). After a stall the offsets of the tiles behind it are
+// wrong, but every store stays in bounds (destinations >= n are skipped, and the
+// slots a pass leaves unwritten keep earlier in-range values), so the context
+// stays usable.
 //
 // Bound: latency of a pass (key loads, ranking, look-back), then L2 for large
 // n. One launch with tiles of 4,096 keys and 512 threads, against a histogram
